@@ -43,6 +43,9 @@ int be_fill_tc_const(void* dst, void* stream);
 // dst[k] = w_N^{k * stride} for k < count, N = 2^logN, forward sign
 int be_fill_pow_tw(void* dst, int elem_bytes, long long count, long long stride, int logN,
                    void* stream);
+// whole 4-step table of a factor 2^logL of an axis 2^logN: entry k * 2^(logN -
+// logL) + i = w_N^{k i}, forward sign
+int be_fill_tw4(void* dst, int elem_bytes, int logL, int logN, void* stream);
 // reference-layout tables of t levels for radix r (r^t - 1 entries)
 int be_fill_ref_tw(int r, int t, double* re, double* im, void* stream);
 int be_round_to_f32(const double* src, float* dst, long long n, void* stream);

@@ -43,6 +43,23 @@ int launch_coltma(const PassDesc& d, int elem_bytes, int b2, long long grid, int
 int launch_plane(const PassDesc& d, int elem_bytes, int b2, long long grid, int threads,
                  size_t smem, void* stream);
 
+// the passes over 8-byte elements (pac_vec.cu, one slice per translation
+// unit): -1 for a pass of another slice
+#define PAC_VEC_DECLARE(k) \
+  int launch_vec_##k(const PassDesc& d, int elem_bytes, int b2, void* stream);
+PAC_VEC_DECLARE(0) PAC_VEC_DECLARE(1) PAC_VEC_DECLARE(2) PAC_VEC_DECLARE(3) PAC_VEC_DECLARE(4)
+PAC_VEC_DECLARE(5) PAC_VEC_DECLARE(6) PAC_VEC_DECLARE(7) PAC_VEC_DECLARE(8) PAC_VEC_DECLARE(9)
+static int launch_vec(const PassDesc& d, int elem_bytes, int b2, void* stream) {
+  static int (*const fn[])(const PassDesc&, int, int, void*) = {
+      launch_vec_0, launch_vec_1, launch_vec_2, launch_vec_3, launch_vec_4,
+      launch_vec_5, launch_vec_6, launch_vec_7, launch_vec_8, launch_vec_9};
+  for (auto f : fn) {
+    const int st = f(d, elem_bytes, b2, stream);
+    if (st >= 0) return st;
+  }
+  return set_error(PAC_ERROR_INTERNAL, "no kernel for a pass over 8-byte elements");
+}
+
 static int cuda_fail(cudaError_t e, const char* what) {
   return set_error(PAC_ERROR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
@@ -300,6 +317,18 @@ __global__ void fill_pow_tw_kernel(Cx<T>* dst, long long count, long long stride
     double sn, cs;
     sincospi(x, &sn, &cs);
     dst[k] = Cx<T>{T(cs), T(sn)};
+  }
+}
+
+template <typename T>
+__global__ void fill_tw4_kernel(Cx<T>* dst, int logL, int logN) {
+  const int logM = logN - logL;
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < (1LL << logN);
+       q += (long long)gridDim.x * blockDim.x) {
+    const long long E = (q >> logM) * (q & ((1LL << logM) - 1));  // below N
+    double sn, cs;
+    sincospi(-2.0 * (double)E / (double)(1LL << logN), &sn, &cs);
+    dst[q] = Cx<T>{T(cs), T(sn)};
   }
 }
 
@@ -853,6 +882,7 @@ static int launch_pipe(const PassDesc& d, int elem_bytes, int b2, long long grid
 
 int be_launch_pass(const PassDesc& d, int elem_bytes, int b2, long long grid, int threads,
                    size_t smem, void* stream) {
+  if (d.vec) return launch_vec(d, elem_bytes, b2, stream);
   if (d.plane) return launch_plane(d, elem_bytes, b2, grid, threads, smem, stream);
   if (d.tma) return launch_coltma(d, elem_bytes, b2, grid, threads, smem, stream);
   if (d.pipe) return launch_pipe(d, elem_bytes, b2, grid, threads, smem, stream);
@@ -916,6 +946,17 @@ int be_fill_pow_tw(void* dst, int elem_bytes, long long count, long long stride,
     fill_pow_tw_kernel<float><<<grid_for(count), 256, 0, (cudaStream_t)stream>>>(
         (Cx<float>*)dst, count, stride, logN);
   PAC_LAUNCHED("fill_pow_tw");
+  return PAC_SUCCESS;
+}
+
+int be_fill_tw4(void* dst, int elem_bytes, int logL, int logN, void* stream) {
+  if (elem_bytes == 8)
+    fill_tw4_kernel<double><<<grid_for(1LL << logN), 256, 0, (cudaStream_t)stream>>>(
+        (Cx<double>*)dst, logL, logN);
+  else
+    fill_tw4_kernel<float><<<grid_for(1LL << logN), 256, 0, (cudaStream_t)stream>>>(
+        (Cx<float>*)dst, logL, logN);
+  PAC_LAUNCHED("fill_tw4");
   return PAC_SUCCESS;
 }
 

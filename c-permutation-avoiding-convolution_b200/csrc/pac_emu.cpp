@@ -395,8 +395,28 @@ static int replay_plane(const PassDesc& d, long long grid) {
   return PAC_SUCCESS;
 }
 
+// the passes over 8-byte elements (pac_emu_vec.cpp, sliced as pac_vec.cu)
+#define PAC_VEC_DECLARE(k) int replay_vec_##k(const PassDesc& d, int elem_bytes, int b2);
+PAC_VEC_DECLARE(0) PAC_VEC_DECLARE(1) PAC_VEC_DECLARE(2) PAC_VEC_DECLARE(3) PAC_VEC_DECLARE(4)
+PAC_VEC_DECLARE(5) PAC_VEC_DECLARE(6) PAC_VEC_DECLARE(7) PAC_VEC_DECLARE(8) PAC_VEC_DECLARE(9)
+static int replay_vec(const PassDesc& d, int elem_bytes, int b2) {
+  static int (*const fn[])(const PassDesc&, int, int) = {
+      replay_vec_0, replay_vec_1, replay_vec_2, replay_vec_3, replay_vec_4,
+      replay_vec_5, replay_vec_6, replay_vec_7, replay_vec_8, replay_vec_9};
+  if (d.W * d.L > 0 && copy_wait_gives_up(d)) return PAC_SUCCESS;
+  for (auto f : fn) {
+    const int st = f(d, elem_bytes, b2);
+    if (st >= 0) return st;
+  }
+  return set_error(PAC_ERROR_INTERNAL, "no replay for a pass over 8-byte elements");
+}
+
 int be_launch_pass(const PassDesc& d, int elem_bytes, int b2, long long grid, int threads,
                    size_t, void*) {
+  if (d.vec) {
+    g_launches++;
+    return replay_vec(d, elem_bytes, b2);
+  }
   if (d.plane) {
 #define PAC_X(T, BY, B2_, L1_, L2_, LC, NT_, MB)                                           \
   if (elem_bytes == BY && b2 == B2_ && d.plane_logN1 == L1_ && d.plane_logN2 == L2_ &&   \
@@ -520,6 +540,18 @@ int be_fill_pow_tw(void* dst, int elem_bytes, long long count, long long stride,
     root((k * stride) & (N - 1), N, &c, &sn);
     if (elem_bytes == 8) put<double>(dst, k, c, sn);
     else put<float>(dst, k, c, sn);
+  }
+  g_launches++;
+  return PAC_SUCCESS;
+}
+
+int be_fill_tw4(void* dst, int elem_bytes, int logL, int logN, void*) {
+  const long long N = 1LL << logN, M = N >> logL;
+  for (long long q = 0; q < N; ++q) {
+    double c, sn;
+    root((q / M) * (q % M), N, &c, &sn);
+    if (elem_bytes == 8) put<double>(dst, q, c, sn);
+    else put<float>(dst, q, c, sn);
   }
   g_launches++;
   return PAC_SUCCESS;

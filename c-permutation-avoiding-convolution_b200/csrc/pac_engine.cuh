@@ -76,6 +76,10 @@ struct PassDesc {
   int tw4_lolog;
   const void* tw4_lo;  // w_N^{0 .. 2^lolog - 1}
   const void* tw4_hi;  // w_N^{k * 2^lolog}
+  const void* tw4_lo64;  // the same two tables in FP64 (pac_vec.cuh)
+  const void* tw4_hi64;
+  const void* tw4_tab;  // or the whole table, in the pass's type (tw4 passes of pac_vec.cuh)
+  int tw4_logN;
   // natural-order store (fft / ifft): this pass is the last factor of its
   // axis group; the earlier factors' lengths are nat_flog[0..nat_nf-1]
   // (outermost first), their product is M = 2^nat_Mlog.
@@ -100,6 +104,8 @@ struct PassDesc {
   // k > 0: column pass staged through shared memory by tensor copies, the
   // k-th geometry of its kind on PAC_COLTMA_LIST (pac_special.h; ColTma)
   int tma;
+  // 1: pass over 8-byte elements (pac_vec.cuh; PAC_VEC_LIST, pac_vec_list.h)
+  int vec;
   // 1: plane pass of a 3D convolution (pac_plane.cuh): axes 1 and 2 of
   // every plane, whose stages are rlog[0 .. plane_n1s-1] (axis 1) then
   // rlog[plane_n1s .. nst-1] (axis 2), on a cluster of 2^logC CTAs
@@ -356,3 +362,4 @@ PAC_HD void nat_line(const PassDesc& d, long long g, long long* in_base, long lo
 #include "pac_stages.cuh"
 #include "pac_coltma.cuh"
 #include "pac_plane.cuh"
+

@@ -39,6 +39,7 @@
 #include "pac.h"
 #include "pac_backend.h"
 #include "pac_special.h"
+#include "pac_vec_list.h"
 
 namespace pac {
 
@@ -91,7 +92,11 @@ struct Schedule {
   struct Tw4 {
     void* lo = nullptr;
     void* hi = nullptr;
+    void* lo64 = nullptr;  // the same in FP64 (FP64 schedules: the same tables)
+    void* hi64 = nullptr;
     int lolog = 0;
+    // whole tables [k][i], keyed by the log of the factor (allocating plans)
+    std::map<int, void*> tab;
   };
   std::map<int, Tw4> tw4;  // keyed by log N
   ~Schedule() {
@@ -100,6 +105,9 @@ struct Schedule {
     for (auto& kv : tw4) {
       be_free(kv.second.lo);
       be_free(kv.second.hi);
+      if (kv.second.lo64 != kv.second.lo) be_free(kv.second.lo64);
+      if (kv.second.hi64 != kv.second.hi) be_free(kv.second.hi64);
+      for (auto& t : kv.second.tab) be_free(t.second);
     }
   }
 };
@@ -153,6 +161,59 @@ static int table_alloc(Arena* ar, void** p, size_t bytes) {
   return *p ? PAC_SUCCESS : set_error(PAC_ERROR_SIZE, "no-allocation scratch too small");
 }
 
+// Plans with the built-in knobs split every axis for the least time in the
+// passes over 8-byte elements.  The costs are microseconds per 2^24 line-unit
+// elements (537 MB moved) measured on HBM-sized arrays, FP64 and FP32 within
+// 15% of each other: fused rows; columns; columns with 4-step twiddles (an
+// outer factor of a split axis).  A column factor costs two passes of a
+// convolution, the innermost factor one; a copy of the same bytes takes 84.
+// Index: log2 of the factor; 0 where no kernel over 8-byte elements exists.
+static const int kCostRow[14] = {0, 0, 0, 0, 0, 100, 96, 98, 98, 123, 130, 144, 162, 230};
+static const int kCostCol[14] = {0, 84, 84, 84, 85, 87, 88, 90, 92, 101, 124, 140, 0, 0};
+static const int kCostTw4[14] = {0, 90, 90, 90, 112, 92, 93, 97, 102, 108, 137, 165, 0, 0};
+
+static bool builtin_split(const Schedule& s) {
+  return !s.tc && s.flog_cap == 0 && s.rlog_cap >= 4 && s.special == 0 && s.w_shift == 0 &&
+         s.plane == 0 && getenv("PAC_MAX_FACTOR_LOG") == nullptr;
+}
+
+// the cheapest split of an axis of 2^lg, digit base 2^b2, into at most three
+// factors; rows: its last factor is the innermost of the plan.  Empty when
+// some factor would have no kernel (short axes, long axes of large bases).
+static std::vector<int> cheapest_split(int lg, int b2, bool rows) {
+  std::vector<int> best, cur;
+  int best_cost = 1 << 30;
+  VecGeo g;
+  auto cost = [&](int f, bool last) {
+    const bool row = rows && last;
+    if (f > 13 || !vec_geometry(b2, row ? MODE_CONV : MODE_DIF, -1, f, row ? 0 : 1, &g)) return 0;
+    return row ? kCostRow[f] : 2 * (last ? kCostCol[f] : kCostTw4[f]);
+  };
+  for (int n = 1; n <= 3; ++n)
+    for (int a = b2; a <= lg; a += b2)
+      for (int b = n > 1 ? b2 : 0; a + b <= lg; b += b2) {
+        const int c = lg - a - b;
+        if ((n == 1 && a != lg) || (n == 2 && (c != 0 || b == 0)) || (n == 3 && c < b2)) {
+          if (n < 2) break;
+          continue;
+        }
+        cur.clear();
+        for (int f : {a, b, c})
+          if (f > 0) cur.push_back(f);
+        int total = 0;
+        for (size_t i = 0; i < cur.size() && total >= 0; ++i) {
+          const int v = cost(cur[i], i + 1 == cur.size());
+          total = v > 0 ? total + v : -1;
+        }
+        if (total > 0 && total < best_cost) {
+          best_cost = total;
+          best = cur;
+        }
+        if (n < 2) break;
+      }
+  return best;
+}
+
 // The factors of every axis and their stage radices -- the one rule every
 // plan follows (allocating plans and the no-allocation entry point alike).
 static int split_axes(Schedule& s, int rank, const int* logs, const int* b2s, int bytes) {
@@ -162,6 +223,12 @@ static int split_axes(Schedule& s, int rank, const int* logs, const int* b2s, in
     int lg = logs[a];
     if (lg == 0) continue;
     const int b2 = b2s[a];
+    if (builtin_split(s)) {
+      const std::vector<int> f = cheapest_split(lg, b2, a == rank - 1);
+      for (size_t i = 0; i < f.size(); ++i)
+        s.vax.push_back({f[i], a, i == 0, i + 1 == f.size(), b2});
+      if (!f.empty()) continue;
+    }
     const int lmax = max_factor_log(bytes, b2, s.flog_cap);
     int digits = lg / b2;
     int dmax = lmax / b2;
@@ -218,19 +285,32 @@ static int build_tables(Schedule& s, Arena* ar, void* stream) {
     if (s.vax[i].last) continue;
     int logN = 0;
     for (size_t j = i; j < s.vax.size() && s.vax[j].axis == s.vax[i].axis; ++j) logN += s.vax[j].log;
-    if (s.tw4.count(logN)) continue;
-    Schedule::Tw4 t;
+    if (!ar && !s.tc && logN <= PAC_TW4_TABLE_LOG) {
+      void*& tab = s.tw4[logN].tab[s.vax[i].log];
+      if (!tab) {
+        PAC_TRY(be_malloc(&tab, (size_t)2 * bytes << logN));
+        PAC_TRY(be_fill_tw4(tab, bytes, s.vax[i].log, logN, stream));
+      }
+    }
+    if (s.tw4[logN].lo) continue;
+    Schedule::Tw4& t = s.tw4[logN];
     t.lolog = (logN + 1) / 2;
     long long nlo = 1LL << t.lolog, nhi = 1LL << (logN - t.lolog);
     PAC_TRY(table_alloc(ar, &t.lo, (size_t)nlo * 2 * bytes));
-    int st = table_alloc(ar, &t.hi, (size_t)nhi * 2 * bytes);
-    if (st != PAC_SUCCESS) {
-      if (!ar) be_free(t.lo);
-      return st;
+    PAC_TRY(table_alloc(ar, &t.hi, (size_t)nhi * 2 * bytes));
+    if (bytes == 8) {
+      t.lo64 = t.lo;
+      t.hi64 = t.hi;
+    } else {
+      PAC_TRY(table_alloc(ar, &t.lo64, (size_t)nlo * 16));
+      PAC_TRY(table_alloc(ar, &t.hi64, (size_t)nhi * 16));
     }
-    s.tw4[logN] = t;
     PAC_TRY(be_fill_pow_tw(t.lo, bytes, nlo, 1, logN, stream));
     PAC_TRY(be_fill_pow_tw(t.hi, bytes, nhi, nlo, logN, stream));
+    if (bytes != 8) {
+      PAC_TRY(be_fill_pow_tw(t.lo64, 8, nlo, 1, logN, stream));
+      PAC_TRY(be_fill_pow_tw(t.hi64, 8, nhi, nlo, logN, stream));
+    }
   }
   return PAC_SUCCESS;
 }
@@ -362,6 +442,11 @@ static PassSpec make_pass(const Schedule& s, int vi, long long batch, long long 
     d.tw4_lolog = t.lolog;
     d.tw4_lo = t.lo;
     d.tw4_hi = t.hi;
+    d.tw4_lo64 = t.lo64;
+    d.tw4_hi64 = t.hi64;
+    auto tab = t.tab.find(v.log);
+    d.tw4_tab = tab == t.tab.end() ? nullptr : tab->second;
+    d.tw4_logN = logN;
   }
   p.grid = d.nlines / d.W;
   p.threads = threads;
@@ -371,11 +456,48 @@ static PassSpec make_pass(const Schedule& s, int vi, long long batch, long long 
   return p;
 }
 
+// Switch a pass to the kernel over 8-byte elements (pac_vec.cuh) of its
+// geometry.  Plans with knobs and the environment's kernel choices keep the
+// kernels those select, the tensor-core form its own; a column tile has to
+// lie within the stride, and the copies want 16-byte aligned arrays.
+static bool apply_vec(const Schedule& s, PassSpec& p) {
+  PassDesc& d = p.d;
+  if (s.special != 0 || s.w_shift != 0 || s.rlog_cap < 4 || d.tc || d.plane) return false;
+  if (getenv("PAC_COLTMA") || getenv("PAC_PIPE") || getenv("PAC_CLUSTER_VARIANT") ||
+      getenv("PAC_SPECIAL_VARIANT"))
+    return false;
+  const int cols = d.logS > 0 ? 1 : 0;
+  VecGeo g;
+  if (!vec_geometry(p.b2, d.mode, d.sign, d.logL, cols, &g)) return false;
+  if (!rads_match(d, d.logL, p.b2, 4)) return false;
+  // 2048-point columns: the pipelined tensor-copy kernel (PAC_COLTMA_LIST)
+  // prefetches through the whole tile (FP64 50 / 45 against 52 / 49 us on
+  // 2048 x 2048, FP32 286 / 268 against 306 / 335 us on 16 of them)
+  if (cols && d.logL == 11 && p.b2 == 1 && !d.nat && d.tw4 == 0 && (d.mode == MODE_DIT || d.sign < 0))
+    return false;
+  if (!cols && d.nat && d.nat_nf > 0) return false;
+  const int logP = s.bytes == 8 ? 0 : 1;  // log2 lines of a unit
+  if (cols && g.logW + logP > d.logS) return false;
+  if (cols && (d.nlines >> d.logS) >= (1LL << 31)) return false;
+  if (((uintptr_t)d.in_re | (uintptr_t)d.in_im | (uintptr_t)d.out_re | (uintptr_t)d.out_im) % 16)
+    return false;
+  d.vec = 1;
+  d.W = 1 << g.logW;
+  d.logW = g.logW;
+  d.nthreads = g.nt;
+  p.threads = g.nt;
+  const long long units = (d.nlines + logP) >> logP;
+  p.grid = g.small ? (units + g.nt - 1) / g.nt : (units + d.W - 1) >> g.logW;
+  p.smem = g.smem;
+  return true;
+}
+
 // Switch a pass to its specialised kernel when pac_special.h has one for its
 // geometry and the tile fits the lines (W divides nlines and the stride).
 static void apply_special(const Schedule& s, PassSpec& p) {
   PassDesc& d = p.d;
   int logW = 0, nt = 0;
+  if (apply_vec(s, p)) return;
   if (d.nat || d.plane) return;
   if (s.special < 0) return;  // tuned off
   // column pass whose tile a CTA cluster shares (W columns within the
@@ -980,9 +1102,9 @@ static int create_plan(pac_plan_t* plan, int rank, const int* dims, const int* d
   p->main.w_shift = knobs.w_shift;
   p->main.plane = knobs.plane;
   int bytes = form == PAC_FORM_F64 ? 8 : 4;
+  p->main.tc = form == PAC_FORM_TC;
   st = build_schedule(p->main, rank, p->logs, b2s, bytes);
   if (st != PAC_SUCCESS) return st;
-  p->main.tc = form == PAC_FORM_TC;
   if (p->main.tc) {
     st = be_malloc(&p->main.tcc, sizeof(TcConst) * TC_CONST_SETS * 32);
     if (st == PAC_SUCCESS) st = be_fill_tc_const(p->main.tcc, nullptr);

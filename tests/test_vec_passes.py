@@ -1,0 +1,66 @@
+"""Passes over 8-byte elements (FP64 lines, FP32 line pairs): every line
+length of the fused rows, the DIF and DIT rows and the columns, at the edges
+of their tiles -- one line, an odd number of lines (the last FP32 pair has
+one), tiles as wide as the stride, outer factors with 4-step twiddles from the
+whole table and (above 2^20 points) from the two-level ones -- against numpy.
+
+Relative L2 errors of an FFT of 2^m points grow with the number of butterfly
+levels; 1e-13 (FP64) and 1e-6 (FP32) are hundreds of roundings at m <= 21."""
+import numpy as np
+import pytest
+
+import parity as P
+from conftest import pac, rng
+
+F64, F32 = pac.PAC_FORM_F64, pac.PAC_FORM_F32
+
+# rows of every length and base (dims, batch, base)
+ROWS = ([((1 << k,), b, 2) for k in range(5, 14) for b in (1, 3)] +
+        [((64,), 67, 2), ((256,), 9, 2), ((512,), 2, 2), ((1024,), 5, 2)] +
+        [((4 ** k,), 5, 4) for k in range(3, 7)] + [((8 ** k,), 5, 8) for k in range(2, 5)])
+# columns of every length and base: at the narrowest stride that has a tile
+# of both types, and one with several tiles
+COLS = ([((1 << k, 256), 1, 2) for k in range(1, 12)] + [((32, 128), 3, 2), ((64, 64), 3, 2),
+        ((128, 32), 3, 2), ((2048, 8), 2, 2), ((512, 16), 1, 2), ((1024, 8), 1, 2)] +
+        [((4 ** k, 64), 2, 4) for k in range(1, 6)] + [((8 ** k, 64), 1, 8) for k in range(1, 4)])
+# split axes: 1D of 2 and 3 factors, long columns, a middle axis, per-axis bases
+SPLIT = [((1 << 14,), 3, 2), ((1 << 15,), 1, 2), ((1 << 17,), 2, 2), ((4 ** 7,), 3, 4),
+         ((8 ** 5,), 2, 8), ((4096, 32), 1, 2), ((4, 4096, 16), 1, 2), ((16, 8192), 1, 2),
+         ((64, 128, 32), 1, (8, 2, 2))]
+LONG = [((1 << 21,), 1, 2)]
+
+
+def check(L, dims, batch, base, form):
+    g = rng(77)
+    shape = (batch,) + dims
+    axes = tuple(range(1, len(shape)))
+    tol = P.TOL if form == F64 else P.TOL_F32
+    x = g.standard_normal(shape) + 1j * g.standard_normal(shape)
+    fx = np.fft.fftn(x, axes=axes)
+    n = int(np.prod(dims))
+    bases = base if isinstance(base, tuple) else (base,) * len(dims)
+    rev = np.ix_(np.arange(batch), *[P.digit_reversal(b, v) for b, v in zip(bases, dims)])
+    want = {pac.OP_AT: fx[rev], pac.OP_CONJ_A: n * np.fft.ifftn(x[rev], axes=axes),
+            pac.OP_FFT: fx, pac.OP_IFFT: np.fft.ifftn(x, axes=axes),
+            pac.OP_UIFFT: np.fft.ifftn(x[rev], axes=axes)}
+    for op, z in want.items():
+        assert P.crel(P.native_transform(L, dims, batch, base, form, op, x), z) < tol, op
+    h = g.standard_normal(dims) + 1j * g.standard_normal(dims)
+    y = P.native_conv(L, dims, batch, base, form, x, h)
+    assert P.crel(y, np.fft.ifftn(fx * np.fft.fftn(h), axes=axes)) < tol
+    h = g.standard_normal(shape) + 1j * g.standard_normal(shape)
+    y = P.native_conv(L, dims, batch, base, form, x, h, per_problem=True)
+    assert P.crel(y, np.fft.ifftn(fx * np.fft.fftn(h, axes=axes), axes=axes)) < tol
+
+
+@pytest.mark.parametrize("form", [F64, F32])
+@pytest.mark.parametrize("dims,batch,base", ROWS + COLS + SPLIT)
+def test_replay(emu, dims, batch, base, form):
+    check(emu, dims, batch, base, form)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", [F64, F32])
+@pytest.mark.parametrize("dims,batch,base", ROWS + COLS + SPLIT + LONG)
+def test_gpu(lib, dims, batch, base, form):
+    check(lib, dims, batch, base, form)
