@@ -53,9 +53,9 @@ void nan_fill(std::vector<CV<V>>& b) {
   }
 }
 
-template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT>
-int go_rows(const PassDesc& d) {
-  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 0, LOGW, NT>;
+template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int OFFS>
+int rows_as(const PassDesc& d) {
+  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 0, LOGW, NT, 0, OFFS>;
   using Real = typename VP::Real;
   std::vector<CV<V>> buf((size_t)VP::TILE);
   V* D = (V*)buf.data();
@@ -67,18 +67,20 @@ int go_rows(const PassDesc& d) {
   for (long long tile = 0; tile < tiles; ++tile) {
     nan_fill<VP>(buf);
     const long long g0 = tile * wl, n = std::min(wl, d.nlines - g0) << LOGL;
-    std::copy_n((const Real*)d.in_re + (g0 << LOGL), n, (Real*)D);
-    std::copy_n((const Real*)d.in_im + (g0 << LOGL), n, (Real*)(D + VP::DIM));
+    for (long long l = 0; l < n >> LOGL; ++l) {
+      const long long o = VP::line_off(d, g0 + l);
+      std::copy_n((const Real*)d.in_re + o, VP::L, (Real*)D + (l << LOGL));
+      std::copy_n((const Real*)d.in_im + o, VP::L, (Real*)(D + VP::DIM) + (l << LOGL));
+    }
     VP::template body<0>(d, tile, buf.data(), tws.data(), ex);
   }
   return PAC_SUCCESS;
 }
 
-template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int TW4>
-int go_cols(const PassDesc& d) {
-  constexpr int DIR = vec_direct(MODE, LOGL, TW4);
+template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int TW4, int DIR, int OFFS>
+int cols_as(const PassDesc& d) {
   constexpr int T = DIR ? NT : (1 << (LOGL + LOGW)) / 16;
-  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 1, LOGW, T, DIR>;
+  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 1, LOGW, T, DIR, OFFS>;
   std::vector<CV<V>> buf((size_t)VP::TILE);
   V* D = (V*)buf.data();
   std::vector<Cx<typename VP::Real>> tws((size_t)VP::TWN + 1);
@@ -101,8 +103,8 @@ int go_cols(const PassDesc& d) {
   const V* iim = (const V*)d.in_im;
   for (long long tile = 0; tile < tiles; ++tile) {
     nan_fill<VP>(buf);
-    int i0, o;
-    VP::tile_coords(d, tile, i0, o);
+    int i0 = 0, o = 0;
+    if (!VP::DIRECT) VP::tile_coords(d, tile, i0, o);
     for (int e = 0; e < VP::L && !VP::DIRECT; ++e)
       for (int w = 0; w < VP::W; ++w) {
         const long long gi = ((long long)o << (LOGL + su)) + ((long long)e << su) + i0 + w;
@@ -114,11 +116,39 @@ int go_cols(const PassDesc& d) {
   return PAC_SUCCESS;
 }
 
+template <int B2, int MODE, int SIGN, int LOGL, int TW4, int OFFS>
+int small_as(const PassDesc& d) {
+  for (long long u = 0; u < d.nlines / VT<V>::LPU; ++u)
+    VecSmall<V, B2, MODE, SIGN, LOGL, OFFS>::template run<TW4>(d, u);
+  return PAC_SUCCESS;
+}
+
+constexpr bool conv_mode(int mode, int sign) {
+  return mode == MODE_CONV || (mode == MODE_DIF && sign < 0) || (mode == MODE_DIT && sign > 0);
+}
+int no_offsets() {
+  return set_error(PAC_ERROR_INTERNAL, "a pass that takes no problem offsets");
+}
+template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT>
+int go_rows(const PassDesc& d) {
+  if (!d.poff) return rows_as<B2, MODE, SIGN, LOGL, LOGW, NT, 0>(d);
+  if constexpr (MODE == MODE_CONV) return rows_as<B2, MODE, SIGN, LOGL, LOGW, NT, 1>(d);
+  else return no_offsets();
+}
+template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int TW4>
+int go_cols(const PassDesc& d) {
+  if (d.poff) {
+    if constexpr (LOGL <= 8 && conv_mode(MODE, SIGN))
+      return cols_as<B2, MODE, SIGN, LOGL, LOGW, NT, TW4, 1, 1>(d);
+    else return no_offsets();
+  }
+  return cols_as<B2, MODE, SIGN, LOGL, LOGW, NT, TW4, vec_direct(MODE, LOGL, TW4), 0>(d);
+}
 template <int B2, int MODE, int SIGN, int LOGL, int TW4>
 int go_small(const PassDesc& d) {
-  for (long long u = 0; u < d.nlines / VT<V>::LPU; ++u)
-    VecSmall<V, B2, MODE, SIGN, LOGL>::template run<TW4>(d, u);
-  return PAC_SUCCESS;
+  if (!d.poff) return small_as<B2, MODE, SIGN, LOGL, TW4, 0>(d);
+  if constexpr (conv_mode(MODE, SIGN)) return small_as<B2, MODE, SIGN, LOGL, TW4, 1>(d);
+  else return no_offsets();
 }
 
 }  // namespace

@@ -42,6 +42,7 @@ namespace pac {
 // ---------------------------------------------------------------------------
 enum PassMode { MODE_DIF = 0, MODE_DIT = 1, MODE_CONV = 2 };
 enum { PAC_MAX_STAGES = 8, PAC_MAX_FACTORS = 4 };
+enum { VEC_RUN = 1, VEC_PREPARE = 2 };
 
 struct PassDesc {
   const void* in_re;
@@ -104,8 +105,14 @@ struct PassDesc {
   // k > 0: column pass staged through shared memory by tensor copies, the
   // k-th geometry of its kind on PAC_COLTMA_LIST (pac_special.h; ColTma)
   int tma;
-  // 1: pass over 8-byte elements (pac_vec.cuh; PAC_VEC_LIST, pac_vec_list.h)
+  // a pass over 8-byte elements (pac_vec.cuh): VEC_RUN; VEC_PREPARE only
+  // loads its kernel and sets its attributes (ahead of a stream capture)
   int vec;
+  // the passes of a batch of equal problems that do not lie back to back
+  // (pac_multi.cpp; vec passes only): element offset of each, the log2 of its
+  // lines; null for a plan's own batch
+  const long long* poff;
+  int logLP;
   // 1: plane pass of a 3D convolution (pac_plane.cuh): axes 1 and 2 of
   // every plane, whose stages are rlog[0 .. plane_n1s-1] (axis 1) then
   // rlog[plane_n1s .. nst-1] (axis 2), on a cluster of 2^logC CTAs

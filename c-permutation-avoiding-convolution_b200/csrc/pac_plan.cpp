@@ -84,6 +84,9 @@ struct Schedule {
   int special = 0;
   int w_shift = 0;
   int plane = 0;        // 3D: 1 plane schedule, -1 line schedule, 0 built-in
+  int whole_tw4 = 1;    // whole 4-step tables for short axes (not for the FP32 forms' FP64
+                        // schedule, which only set-up uses)
+  int short_cols = 0;   // columns of at most 256 points (batches of problems at any offset)
   void* tcc = nullptr;  // its DFT operand table (tensor-core form)
   std::vector<VAx> vax;
   std::vector<std::vector<int>> rad;  // per factor: stage radix logs, DIF order
@@ -180,13 +183,13 @@ static bool builtin_split(const Schedule& s) {
 // the cheapest split of an axis of 2^lg, digit base 2^b2, into at most three
 // factors; rows: its last factor is the innermost of the plan.  Empty when
 // some factor would have no kernel (short axes, long axes of large bases).
-static std::vector<int> cheapest_split(int lg, int b2, bool rows) {
+static std::vector<int> cheapest_split(int lg, int b2, bool rows, bool short_cols) {
   std::vector<int> best, cur;
   int best_cost = 1 << 30;
   VecGeo g;
   auto cost = [&](int f, bool last) {
     const bool row = rows && last;
-    if (f > 13 || !vec_geometry(b2, row ? MODE_CONV : MODE_DIF, -1, f, row ? 0 : 1, &g)) return 0;
+    if (f > 13 || (short_cols && !row && f > 8) || !vec_geometry(b2, row ? MODE_CONV : MODE_DIF, -1, f, row ? 0 : 1, &g)) return 0;
     return row ? kCostRow[f] : 2 * (last ? kCostCol[f] : kCostTw4[f]);
   };
   for (int n = 1; n <= 3; ++n)
@@ -224,7 +227,7 @@ static int split_axes(Schedule& s, int rank, const int* logs, const int* b2s, in
     if (lg == 0) continue;
     const int b2 = b2s[a];
     if (builtin_split(s)) {
-      const std::vector<int> f = cheapest_split(lg, b2, a == rank - 1);
+      const std::vector<int> f = cheapest_split(lg, b2, a == rank - 1, s.short_cols);
       for (size_t i = 0; i < f.size(); ++i)
         s.vax.push_back({f[i], a, i == 0, i + 1 == f.size(), b2});
       if (!f.empty()) continue;
@@ -285,7 +288,7 @@ static int build_tables(Schedule& s, Arena* ar, void* stream) {
     if (s.vax[i].last) continue;
     int logN = 0;
     for (size_t j = i; j < s.vax.size() && s.vax[j].axis == s.vax[i].axis; ++j) logN += s.vax[j].log;
-    if (!ar && !s.tc && logN <= PAC_TW4_TABLE_LOG) {
+    if (!ar && !s.tc && s.whole_tw4 && logN <= PAC_TW4_TABLE_LOG) {
       void*& tab = s.tw4[logN].tab[s.vax[i].log];
       if (!tab) {
         PAC_TRY(be_malloc(&tab, (size_t)2 * bytes << logN));
@@ -481,7 +484,7 @@ static bool apply_vec(const Schedule& s, PassSpec& p) {
   if (cols && (d.nlines >> d.logS) >= (1LL << 31)) return false;
   if (((uintptr_t)d.in_re | (uintptr_t)d.in_im | (uintptr_t)d.out_re | (uintptr_t)d.out_im) % 16)
     return false;
-  d.vec = 1;
+  d.vec = VEC_RUN;
   d.W = 1 << g.logW;
   d.logW = g.logW;
   d.nthreads = g.nt;
@@ -847,14 +850,15 @@ static PassSpec make_plane_pass(const Schedule& s, long long batch, long long N)
 static void build_conv_passes(pac_plan_s* pl, const void* x_re, const void* x_im,
                               const void* h_re, const void* h_im, int per_problem, void* y_re,
                               void* y_im, double scale, std::vector<PassSpec>& passes,
-                              bool allow_plane = true) {
+                              bool allow_plane = true, long long copies = 0) {
   const Schedule& s = pl->main;
+  const long long batch = copies ? copies : pl->batch;
   const long long N = pl->N;
   const int m = (int)s.vax.size();
   const long long hmask = per_problem ? -1LL : (N - 1);
   if (allow_plane && plane_active(s)) {
     // DIF axis 0, the plane pass, DIT axis 0
-    PassSpec a = make_pass(s, 0, pl->batch, N);
+    PassSpec a = make_pass(s, 0, batch, N);
     a.d.mode = MODE_DIF;
     a.d.sign = -1;
     a.d.in_re = x_re;
@@ -862,7 +866,7 @@ static void build_conv_passes(pac_plan_s* pl, const void* x_re, const void* x_im
     a.d.out_re = y_re;
     a.d.out_im = y_im;
     passes.push_back(a);
-    PassSpec p = make_plane_pass(s, pl->batch, N);
+    PassSpec p = make_plane_pass(s, batch, N);
     p.d.mode = MODE_CONV;
     p.d.h_re = h_re;
     p.d.h_im = h_im;
@@ -873,7 +877,7 @@ static void build_conv_passes(pac_plan_s* pl, const void* x_re, const void* x_im
     p.d.out_re = y_re;
     p.d.out_im = y_im;
     passes.push_back(p);
-    PassSpec c = make_pass(s, 0, pl->batch, N);
+    PassSpec c = make_pass(s, 0, batch, N);
     c.d.mode = MODE_DIT;
     c.d.sign = +1;
     c.d.in_re = y_re;
@@ -884,7 +888,7 @@ static void build_conv_passes(pac_plan_s* pl, const void* x_re, const void* x_im
     return;
   }
   for (int vi = 0; vi < m - 1; ++vi) {
-    PassSpec p = make_pass(s, vi, pl->batch, N);
+    PassSpec p = make_pass(s, vi, batch, N);
     p.d.mode = MODE_DIF;
     p.d.sign = -1;
     p.d.tw4 = s.vax[vi].last ? 0 : 1;
@@ -895,7 +899,7 @@ static void build_conv_passes(pac_plan_s* pl, const void* x_re, const void* x_im
     passes.push_back(p);
   }
   {
-    PassSpec p = make_pass(s, m - 1, pl->batch, N);
+    PassSpec p = make_pass(s, m - 1, batch, N);
     p.d.mode = MODE_CONV;
     p.d.h_re = h_re;
     p.d.h_im = h_im;
@@ -908,7 +912,7 @@ static void build_conv_passes(pac_plan_s* pl, const void* x_re, const void* x_im
     passes.push_back(p);
   }
   for (int vi = m - 2; vi >= 0; --vi) {
-    PassSpec p = make_pass(s, vi, pl->batch, N);
+    PassSpec p = make_pass(s, vi, batch, N);
     p.d.mode = MODE_DIT;
     p.d.sign = +1;
     p.d.tw4 = s.vax[vi].last ? 0 : 2;
@@ -949,6 +953,35 @@ int plan_conv_descs(pac_plan_s* pl, const void* x_re, const void* x_im, const vo
     descs.push_back(p.d);
     ctas.push_back(p.grid);
     smem.push_back(p.smem);
+  }
+  return PAC_SUCCESS;
+}
+// For a batch of plans: the convolution passes of `copies` problems of the
+// plan's shape at element offsets poff[0 ..] (device array) of packed arrays,
+// a filter spectrum each.  Empty when some pass has no kernel that takes
+// such offsets.
+int plan_batch_passes(pac_plan_s* pl, long long copies, const long long* poff, const void* x_re,
+                      const void* x_im, const void* h_re, const void* h_im, void* y_re,
+                      void* y_im, std::vector<PassDesc>& descs, std::vector<long long>& tiles) {
+  const Schedule& s = pl->main;
+  descs.clear();
+  tiles.clear();
+  if (s.vax.empty()) return PAC_SUCCESS;
+  std::vector<PassSpec> passes;
+  build_conv_passes(pl, x_re, x_im, h_re, h_im, 1, y_re, y_im, 1.0, passes, false, copies);
+  int logN = 0;
+  for (const VAx& v : s.vax) logN += v.log;
+  for (auto& p : passes) {
+    if (!apply_vec(s, p) || (p.d.logS > 0 && p.d.logL > 8)) {
+      descs.clear();
+      tiles.clear();
+      return PAC_SUCCESS;
+    }
+    p.d.poff = poff;
+    p.d.logLP = logN - p.d.logL;
+    p.d.status = pl->status;
+    descs.push_back(p.d);
+    tiles.push_back(p.grid);
   }
   return PAC_SUCCESS;
 }
@@ -1053,7 +1086,7 @@ bool tune_from_env_cache(int rank, const int* dims, const int* bases, int batch,
 extern "C" {
 
 static int create_plan(pac_plan_t* plan, int rank, const int* dims, const int* digit_bases,
-                       int batch, int form, const pac_tune_t* tune) {
+                       int batch, int form, const pac_tune_t* tune, int short_cols = 0) {
   if (!plan || !dims || !digit_bases || rank < 1 || rank > 3 || batch < 1)
     return set_error(PAC_ERROR_INVALID_VALUE, "pac_plan_create: invalid rank/dims/batch");
   const pac_tune_t knobs = tune ? *tune : pac_tune_t{0, 0, 0, 0, 0};
@@ -1101,6 +1134,7 @@ static int create_plan(pac_plan_t* plan, int rank, const int* dims, const int* d
   p->main.special = knobs.special;
   p->main.w_shift = knobs.w_shift;
   p->main.plane = knobs.plane;
+  p->main.short_cols = short_cols;
   int bytes = form == PAC_FORM_F64 ? 8 : 4;
   p->main.tc = form == PAC_FORM_TC;
   st = build_schedule(p->main, rank, p->logs, b2s, bytes);
@@ -1112,6 +1146,7 @@ static int create_plan(pac_plan_t* plan, int rank, const int* dims, const int* d
   }
   if (bytes != 8) {
     p->s64.reset(new Schedule());
+    p->s64->whole_tw4 = 0;
     st = build_schedule(*p->s64, rank, p->logs, b2s, 8);
     if (st != PAC_SUCCESS) return st;
   }
@@ -1143,6 +1178,20 @@ PAC_API int pac_plan_create(pac_plan_t* plan, int rank, const int* dims, int bat
   const int bases[3] = {digit_base, digit_base, digit_base};
   return pac_plan_create_axes(plan, rank, dims, bases, batch, form);
 }
+
+}  // extern "C"
+namespace pac {
+// a multi-plan's plan of one shape: the built-in knobs (or the cached ones),
+// factors whose passes can serve problems at any offset
+int plan_create_for_batch(pac_plan_t* plan, int rank, const int* dims, const int* bases,
+                          int form) {
+  pac_tune_t t;
+  if (tune_from_env_cache(rank, dims, bases, 1, form, &t))
+    return create_plan(plan, rank, dims, bases, 1, form, &t);
+  return create_plan(plan, rank, dims, bases, 1, form, nullptr, 1);
+}
+}  // namespace pac
+extern "C" {
 
 PAC_API int pac_plan_destroy(pac_plan_t plan) {
   delete plan;

@@ -79,14 +79,14 @@ int col_map(CUtensorMap* m, const void* base, const PassDesc& d) {
   return PAC_SUCCESS;
 }
 
-template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int MINB>
-int go_rows(const PassDesc& d, cudaStream_t st) {
-  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 0, LOGW, NT>;
+template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int MINB, int OFFS>
+int rows_as(const PassDesc& d, cudaStream_t st) {
+  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 0, LOGW, NT, 0, OFFS>;
   static Resident res;
-  auto kern = pac_vec_rows_kernel<V, B2, MODE, SIGN, LOGL, LOGW, NT, MINB>;
+  auto kern = pac_vec_rows_kernel<V, B2, MODE, SIGN, LOGL, LOGW, NT, MINB, OFFS>;
   long long slots = 0;
   int s = resident(res, kern, NT, VP::SMEM + 128, &slots);
-  if (s != PAC_SUCCESS) return s;
+  if (s != PAC_SUCCESS || d.vec == VEC_PREPARE) return s;
   const long long wl = VP::W * VP::LPU, tiles = (d.nlines + wl - 1) / wl;
   kern<<<(unsigned)(tiles < slots ? tiles : slots), NT, VP::SMEM + 128, st>>>(d);
   PAC_CU(cudaGetLastError(), "pac_vec_rows_kernel launch");
@@ -94,41 +94,89 @@ int go_rows(const PassDesc& d, cudaStream_t st) {
   return PAC_SUCCESS;
 }
 
-template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int MINB, int TW4>
-int go_cols(const PassDesc& d, cudaStream_t st) {
+// column tiles read straight from global memory
+template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int MINB, int TW4, int OFFS>
+int cols_direct(const PassDesc& d, cudaStream_t st) {
+  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 1, LOGW, NT, 1, OFFS>;
   static Resident res;
+  auto kern = pac_vec_direct_kernel<V, B2, MODE, SIGN, LOGL, LOGW, NT, MINB, TW4, OFFS>;
   long long slots = 0;
-  int s = 0;
-  const long long tiles = (d.nlines / VT<V>::LPU) >> LOGW;
-  if constexpr (vec_direct(MODE, LOGL, TW4)) {
-    using VP = VecPass<V, B2, MODE, SIGN, LOGL, 1, LOGW, NT, 1>;
-    auto kern = pac_vec_direct_kernel<V, B2, MODE, SIGN, LOGL, LOGW, NT, MINB, TW4>;
-    if ((s = resident(res, kern, NT, VP::TILE_BYTES, &slots)) != PAC_SUCCESS) return s;
-    if (tiles > 0x7fffffffLL) return set_error(PAC_ERROR_SIZE, "pass grid too large");
-    kern<<<(unsigned)tiles, NT, VP::TILE_BYTES, st>>>(d);
-  } else {
-    constexpr int T = (1 << (LOGL + LOGW)) / 16, MB = 512 / T;
-    using VP = VecPass<V, B2, MODE, SIGN, LOGL, 1, LOGW, T>;
-    auto kern = pac_vec_cols_kernel<V, B2, MODE, SIGN, LOGL, LOGW, T, MB, TW4>;
-    if ((s = resident(res, kern, T, VP::SMEM + 128, &slots)) != PAC_SUCCESS) return s;
-    CUtensorMap m[2];
-    if ((s = col_map<VP>(&m[0], d.in_re, d)) != PAC_SUCCESS) return s;
-    if ((s = col_map<VP>(&m[1], d.in_im, d)) != PAC_SUCCESS) return s;
-    kern<<<(unsigned)(tiles < slots ? tiles : slots), T, VP::SMEM + 128, st>>>(d, m[0], m[1]);
-  }
-  PAC_CU(cudaGetLastError(), "column pass over 8-byte elements");
+  int s = resident(res, kern, NT, VP::TILE_BYTES, &slots);
+  if (s != PAC_SUCCESS || d.vec == VEC_PREPARE) return s;
+  const long long tiles = (d.nlines / VP::LPU) >> LOGW;
+  if (tiles > 0x7fffffffLL) return set_error(PAC_ERROR_SIZE, "pass grid too large");
+  kern<<<(unsigned)tiles, NT, VP::TILE_BYTES, st>>>(d);
+  PAC_CU(cudaGetLastError(), "pac_vec_direct_kernel launch");
   count_launch();
   return PAC_SUCCESS;
 }
 
-template <int B2, int MODE, int SIGN, int LOGL, int TW4>
-int go_small(const PassDesc& d, cudaStream_t st) {
+// column tiles brought in by tensor copies, 16 elements a thread
+template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int TW4>
+int cols_copied(const PassDesc& d, cudaStream_t st) {
+  constexpr int T = (1 << (LOGL + LOGW)) / 16, MB = 512 / T;
+  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 1, LOGW, T>;
+  static Resident res;
+  auto kern = pac_vec_cols_kernel<V, B2, MODE, SIGN, LOGL, LOGW, T, MB, TW4>;
+  long long slots = 0;
+  int s = resident(res, kern, T, VP::SMEM + 128, &slots);
+  if (s != PAC_SUCCESS || d.vec == VEC_PREPARE) return s;
+  CUtensorMap m[2];
+  if ((s = col_map<VP>(&m[0], d.in_re, d)) != PAC_SUCCESS) return s;
+  if ((s = col_map<VP>(&m[1], d.in_im, d)) != PAC_SUCCESS) return s;
+  const long long tiles = (d.nlines / VP::LPU) >> LOGW;
+  kern<<<(unsigned)(tiles < slots ? tiles : slots), T, VP::SMEM + 128, st>>>(d, m[0], m[1]);
+  PAC_CU(cudaGetLastError(), "pac_vec_cols_kernel launch");
+  count_launch();
+  return PAC_SUCCESS;
+}
+
+template <int B2, int MODE, int SIGN, int LOGL, int TW4, int OFFS>
+int small_as(const PassDesc& d, cudaStream_t st) {
   const long long grid = (d.nlines / VT<V>::LPU + 255) / 256;
   if (grid > 0x7fffffffLL) return set_error(PAC_ERROR_SIZE, "pass grid too large");
-  pac_vec_small_kernel<V, B2, MODE, SIGN, LOGL, TW4><<<(unsigned)grid, 256, 0, st>>>(d);
+  auto kern = pac_vec_small_kernel<V, B2, MODE, SIGN, LOGL, TW4, OFFS>;
+  if (d.vec == VEC_PREPARE) {
+    cudaFuncAttributes fa;
+    PAC_CU(cudaFuncGetAttributes(&fa, kern), "cudaFuncGetAttributes");
+    return PAC_SUCCESS;
+  }
+  kern<<<(unsigned)grid, 256, 0, st>>>(d);
   PAC_CU(cudaGetLastError(), "pac_vec_small_kernel launch");
   count_launch();
   return PAC_SUCCESS;
+}
+
+// problems at any offset: convolutions only
+constexpr bool conv_mode(int mode, int sign) {
+  return mode == MODE_CONV || (mode == MODE_DIF && sign < 0) || (mode == MODE_DIT && sign > 0);
+}
+int no_offsets() {
+  return set_error(PAC_ERROR_INTERNAL, "a pass that takes no problem offsets");
+}
+
+template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int MINB>
+int go_rows(const PassDesc& d, cudaStream_t st) {
+  if (!d.poff) return rows_as<B2, MODE, SIGN, LOGL, LOGW, NT, MINB, 0>(d, st);
+  if constexpr (MODE == MODE_CONV) return rows_as<B2, MODE, SIGN, LOGL, LOGW, NT, MINB, 1>(d, st);
+  else return no_offsets();
+}
+template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int MINB, int TW4>
+int go_cols(const PassDesc& d, cudaStream_t st) {
+  if (d.poff) {
+    if constexpr (LOGL <= 8 && conv_mode(MODE, SIGN))
+      return cols_direct<B2, MODE, SIGN, LOGL, LOGW, NT, MINB, TW4, 1>(d, st);
+    else return no_offsets();
+  }
+  if constexpr (vec_direct(MODE, LOGL, TW4))
+    return cols_direct<B2, MODE, SIGN, LOGL, LOGW, NT, MINB, TW4, 0>(d, st);
+  else return cols_copied<B2, MODE, SIGN, LOGL, LOGW, TW4>(d, st);
+}
+template <int B2, int MODE, int SIGN, int LOGL, int TW4>
+int go_small(const PassDesc& d, cudaStream_t st) {
+  if (!d.poff) return small_as<B2, MODE, SIGN, LOGL, TW4, 0>(d, st);
+  if constexpr (conv_mode(MODE, SIGN)) return small_as<B2, MODE, SIGN, LOGL, TW4, 1>(d, st);
+  else return no_offsets();
 }
 
 }  // namespace

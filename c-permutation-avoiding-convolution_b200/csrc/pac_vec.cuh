@@ -460,10 +460,24 @@ PAC_HD void vtw4_apply(const PassDesc& d, long long g0, int blk, int logL, CV<V>
   });
 }
 
+// offset, in units, of column unit u's first element
+template <int LOGL, int LPU, int OFFS>
+PAC_HD long long unit_base(const PassDesc& d, long long u) {
+  const int su = d.logS - ilog2(LPU);
+  long long b = 0;
+  if constexpr (OFFS != 0) {
+    const int lp = d.logLP - ilog2(LPU);
+    b = d.poff[u >> lp] >> ilog2(LPU);
+    u &= (1LL << lp) - 1;
+  }
+  return b + ((u >> su) << (LOGL + su)) + (u & ((1LL << su) - 1));
+}
+
 // ---------------------------------------------------------------------------
 // The pass
 // ---------------------------------------------------------------------------
-template <class V, int B2, int MODE, int SIGN, int LOGL, int COLS, int LOGW, int NT, int DIR = 0>
+template <class V, int B2, int MODE, int SIGN, int LOGL, int COLS, int LOGW, int NT, int DIR = 0,
+          int OFFS = 0>
 struct VecPass {
   using Real = typename VT<V>::Real;
   using RS = RadsFor<LOGL, B2>;
@@ -613,9 +627,7 @@ struct VecPass {
     constexpr int I = stage_at(0), LR = RS::v[I], R = 1 << LR;
     constexpr int logell = RS::logK(LOGL, I) - LR;
     const int rowsh = d.logS - ilog2(LPU);
-    int i0, o;
-    tile_coords(d, tile, i0, o);
-    const long long base = ((long long)o << (LOGL + rowsh)) + i0;
+    const long long base = tile_base(d, tile);
     const V* ire = (const V*)d.in_re;
     const V* iim = (const V*)d.in_im;
     static_for<TPT / R>([&](auto kk) {
@@ -701,9 +713,9 @@ struct VecPass {
     const int blk = e0 >> VIN;
     const long long l0 = ((tile << LOGW) + w) * LPU;
     const long long last = d.nlines - 1;
-    const long long h0 = (((l0 < last ? l0 : last) << LOGL) & d.h_mask) + blk;
+    const long long h0 = (line_off(d, l0 < last ? l0 : last) & d.h_mask) + blk;
     const long long h1 =
-        LPU == 2 ? (((l0 + 1 < last ? l0 + 1 : last) << LOGL) & d.h_mask) + blk : h0;
+        LPU == 2 ? (line_off(d, l0 + 1 < last ? l0 + 1 : last) & d.h_mask) + blk : h0;
     static_for<GF>([&](auto ff) {
       constexpr int off = drev_c(freq<Q, ff.value>(), VIN, B2) << (LOGL - VIN);
       if constexpr (LPU == 1) {
@@ -803,6 +815,13 @@ struct VecPass {
     });
   }
 
+  // element offset of row l (OFFS: of problems that do not lie back to back,
+  // PassDesc.poff; a variant of its own, as the look-up cost the others 4%)
+  static PAC_HD long long line_off(const PassDesc& d, long long l) {
+    if constexpr (!OFFS) return l << LOGL;
+    return d.poff[l >> d.logLP] + ((l & ((1LL << d.logLP) - 1)) << LOGL);
+  }
+
   // ---- DIT rows: the dense tile through registers into the padded layout --
   static PAC_HD void relay_read(int t, const CV<V>* B, CV<V> (&x)[TPT]) {
     const V* D = reinterpret_cast<const V*>(B);
@@ -822,12 +841,15 @@ struct VecPass {
   // rows: the unit's line(s) in the output, and which of them exist
   struct RowOut {
     Real *re, *im;
+    long long next;  // from the first line to the second
     bool first, second;
   };
   static PAC_HD RowOut row_out(const PassDesc& d, long long tile, int w, int e0) {
     const long long l0 = ((tile << LOGW) + w) * LPU;
-    const long long o = (l0 << LOGL) + e0;
-    return {(Real*)d.out_re + o, (Real*)d.out_im + o, l0 < d.nlines, l0 + 1 < d.nlines};
+    const bool first = l0 < d.nlines, second = LPU == 2 && l0 + 1 < d.nlines;
+    const long long o = !OFFS || first ? line_off(d, l0) + e0 : 0;
+    const long long next = OFFS && second ? line_off(d, l0 + 1) + e0 - o : L;
+    return {(Real*)d.out_re + o, (Real*)d.out_im + o, next, first, second};
   }
   static PAC_HD void put_row(const RowOut& r, int off, CV<V> v) {
     if constexpr (LPU == 1) {
@@ -844,8 +866,8 @@ struct VecPass {
         r.im[off] = c;
       }
       if (r.second) {
-        r.re[off + L] = b;
-        r.im[off + L] = e;
+        r.re[r.next + off] = b;
+        r.im[r.next + off] = e;
       }
     }
   }
@@ -855,6 +877,10 @@ struct VecPass {
     const int logSU = d.logS - ilog2(LPU);
     i0 = (int)(g0 & ((1LL << logSU) - 1));
     o = (int)(g0 >> logSU);
+  }
+  // unit offset of a column tile's first row
+  static PAC_HD long long tile_base(const PassDesc& d, long long tile) {
+    return unit_base<LOGL, LPU, OFFS>(d, tile << LOGW);
   }
   // the last step's outputs from the registers to global memory: whole rows
   // of W elements (columns; at their natural index when the pass ends a
@@ -871,15 +897,13 @@ struct VecPass {
     long long base = 0;
     int rowsh = d.logS - ilog2(LPU);
     if constexpr (COLS) {
-      int i0, o;
-      tile_coords(d, tile, i0, o);
       if (d.nat) {
         long long in_base, out_base;
         nat_line<B2>(d, (tile << LOGW) * LPU, &in_base, &out_base);
         base = out_base >> ilog2(LPU);
         rowsh += d.nat_Mlog;
       } else {
-        base = ((long long)o << (LOGL + rowsh)) + i0;
+        base = tile_base(d, tile);
       }
     }
     static_for<TPT / R>([&](auto kk) {
@@ -960,7 +984,7 @@ struct VecPass {
 };
 
 // Columns of 2 to 16 elements: one unit a thread, registers only.
-template <class V, int B2, int MODE, int SIGN, int LOGL>
+template <class V, int B2, int MODE, int SIGN, int LOGL, int OFFS = 0>
 struct VecSmall {
   static constexpr int L = 1 << LOGL, LPU = VT<V>::LPU;
   static_assert(LOGL >= 1 && LOGL <= 4 && LOGL % B2 == 0 && (B2 != 3 || LOGL == 3), "one stage");
@@ -972,7 +996,7 @@ struct VecSmall {
     const V* iim = (const V*)d.in_im;
     V* ore = (V*)d.out_re;
     V* oim = (V*)d.out_im;
-    const long long in0 = ((u >> su) << (LOGL + su)) + (u & ((1LL << su) - 1));
+    const long long in0 = unit_base<LOGL, LPU, OFFS>(d, u);
     long long out0 = in0;
     int osh = su;
     if (MODE == MODE_DIF && d.nat) {

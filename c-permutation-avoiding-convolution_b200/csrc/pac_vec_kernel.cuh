@@ -89,9 +89,10 @@ __device__ __forceinline__ void vec_tiles(const PassDesc& d, CV<V>* B, uint64_t*
   }
 }
 
-template <class V, int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int MINB>
+template <class V, int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int MINB,
+          int OFFS>
 __global__ void __launch_bounds__(NT, MINB) pac_vec_rows_kernel(const __grid_constant__ PassDesc d) {
-  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 0, LOGW, NT>;
+  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 0, LOGW, NT, 0, OFFS>;
   using Real = typename VP::Real;
   extern __shared__ unsigned char pac_smem_raw[];
   __shared__ __align__(8) uint64_t bar;
@@ -105,6 +106,16 @@ __global__ void __launch_bounds__(NT, MINB) pac_vec_rows_kernel(const __grid_con
     const long long n = d.nlines - g0 < WL ? d.nlines - g0 : WL;
     const uint32_t bytes = (uint32_t)(n << LOGL) * (uint32_t)sizeof(Real);
     mbar_arrive_expect_tx(&bar, 2 * bytes);
+    if constexpr (OFFS) {  // line by line
+      for (int l = 0; l < (int)n; ++l) {
+        const long long o = VP::line_off(d, g0 + l);
+        Real* dst = (Real*)D + (l << LOGL);
+        bulk_load(dst, (const Real*)d.in_re + o, (uint32_t)sizeof(Real) << LOGL, &bar);
+        bulk_load(dst + VP::LPU * VP::DIM, (const Real*)d.in_im + o, (uint32_t)sizeof(Real) << LOGL,
+                  &bar);
+      }
+      return;
+    }
     bulk_load(D, (const Real*)d.in_re + (g0 << LOGL), bytes, &bar);
     bulk_load(D + VP::DIM, (const Real*)d.in_im + (g0 << LOGL), bytes, &bar);
   };
@@ -151,9 +162,10 @@ struct VecExecOnce {
   __device__ __forceinline__ void sync() { vec_sync<VP::kThreads>(); }
   __device__ __forceinline__ void freed() {}
 };
-template <class V, int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int MINB, int TW4>
+template <class V, int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int MINB, int TW4,
+          int OFFS>
 __global__ void __launch_bounds__(NT, MINB) pac_vec_direct_kernel(const __grid_constant__ PassDesc d) {
-  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 1, LOGW, NT, 1>;
+  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 1, LOGW, NT, 1, OFFS>;
   using Real = typename VP::Real;
   extern __shared__ __align__(16) unsigned char pac_smem_raw[];
   CV<V>* B = reinterpret_cast<CV<V>*>(pac_smem_raw);
@@ -161,10 +173,10 @@ __global__ void __launch_bounds__(NT, MINB) pac_vec_direct_kernel(const __grid_c
   VP::template body<TW4>(d, blockIdx.x, B, (const Cx<Real>*)nullptr, ex);
 }
 
-template <class V, int B2, int MODE, int SIGN, int LOGL, int TW4>
+template <class V, int B2, int MODE, int SIGN, int LOGL, int TW4, int OFFS>
 __global__ void __launch_bounds__(256) pac_vec_small_kernel(const __grid_constant__ PassDesc d) {
   const long long u = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (u < d.nlines / VT<V>::LPU) VecSmall<V, B2, MODE, SIGN, LOGL>::template run<TW4>(d, u);
+  if (u < d.nlines / VT<V>::LPU) VecSmall<V, B2, MODE, SIGN, LOGL, OFFS>::template run<TW4>(d, u);
 }
 
 }  // namespace pac

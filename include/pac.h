@@ -248,19 +248,22 @@ PAC_API int pac_convolve_1d_noalloc(const double* x_re, const double* x_im, cons
  * in the problem's own row-major layout.  Problems of one shape share their
  * plan and twiddles.
  *
- * pac_multi_convolve runs every problem's convolution passes level by level
- * (level k = the k-th pass of every problem that has one): a level is one
- * persistent launch whose CTAs take work items (pass, tile) from a device
- * work queue, largest tiles first, so small and large problems share the
- * GPU -- or two such launches side by side when the level mixes tiles of
- * more and less than 72 KB of shared memory.  With a non-NULL stream the
- * launches are captured once into a CUDA graph per set of buffer addresses
- * and replayed afterwards (the first call for new addresses captures; later
- * calls launch the graph).  Calls on one multi-plan are serialised by a
- * lock on the host, but its work-queue counters are one device block per
- * multi-plan: calls whose device work overlaps (different streams, or graph
- * replays on different streams) take items from the same counters and
- * corrupt each other's results.  Queue the calls of one multi-plan on one
+ * pac_multi_convolve launches every pass of a shape once for all problems
+ * of that shape; the shapes are independent of each other and share the GPU
+ * over a few streams of the multi-plan, forked from the caller's and joined
+ * back into it.  Shapes whose passes have no such kernel (explicit knobs,
+ * the tensor-core form, strides narrower than a column tile, problems that do
+ * not start at a multiple of 16 bytes) run level by level instead (level k =
+ * the k-th pass of every such problem): a level is one persistent launch
+ * whose CTAs take work items (pass, tile) from a device work queue, largest
+ * tiles first, or two such launches side by side when the level mixes tiles
+ * of more and less than 72 KB of shared memory.  With a non-NULL stream the
+ * launches of a set of buffer addresses are captured into a CUDA graph at
+ * its second call and replayed from then on.  Calls on one multi-plan are
+ * serialised by a lock on the host, but its streams and its work-queue
+ * counters (one device block) are the multi-plan's own: calls whose device
+ * work overlaps (different streams, or graph replays on different streams)
+ * take items from the same counters and corrupt each other's results.  Queue the calls of one multi-plan on one
  * stream, or use one multi-plan per stream. */
 typedef struct pac_multi_s* pac_multi_t;
 
@@ -284,8 +287,8 @@ PAC_API int pac_multi_convolve(pac_multi_t multi, const void* x_re, const void* 
 typedef struct {
   int nprob;
   int nshapes;            /* distinct shapes (plans) */
-  int nlevels;            /* levels of passes per pac_multi_convolve */
-  long long items[8];     /* work items (CTAs) of each level */
+  int nlevels;            /* levels of passes per pac_multi_convolve (8 at most are told) */
+  long long items[8];     /* tiles of each level */
   long long elements;     /* total elements of one packed array */
   int graph;              /* 1 once a CUDA graph replays the levels */
   double level_ms[8];     /* per-level mean time of the timed calls */

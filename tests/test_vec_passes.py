@@ -53,6 +53,29 @@ def check(L, dims, batch, base, form):
     assert P.crel(y, np.fft.ifftn(fx * np.fft.fftn(h, axes=axes), axes=axes)) < tol
 
 
+# uneven batches: problems of one shape apart from each other (an odd number
+# of them, so the last FP32 pair of rows has one line), every short-column
+# length, and two-element problems after which nothing starts at a multiple of
+# 16 bytes (those take the work queue)
+UNEVEN = [[(256,), (64, 32), (256,), (2 ** 14,), (512,), (256,), (2 ** 14,), (8192,), (64, 32)],
+          [(1 << k, 256) for k in range(1, 9)] + [(2 ** 15,), (4, 8, 256), (2 ** 15,), (1024, 64)],
+          [(256,), (2048,), (2,), (256,), (2048,), (64, 64), (2,), (2,), (2,), (256,)]]
+
+
+@pytest.mark.parametrize("form", [F64, F32])
+@pytest.mark.parametrize("shapes", UNEVEN)
+def test_uneven_replay(emu, shapes, form):
+    P.check_multi(emu, shapes, form)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("stream", [False, True])
+@pytest.mark.parametrize("form", [F64, F32])
+@pytest.mark.parametrize("shapes", UNEVEN + [[(2 ** 20,), (256,), (2048, 512), (2 ** 20,), (256,)]])
+def test_uneven_gpu(lib, shapes, form, stream):
+    P.check_multi(lib, shapes, form, stream=stream)
+
+
 @pytest.mark.parametrize("form", [F64, F32])
 @pytest.mark.parametrize("dims,batch,base", ROWS + COLS + SPLIT)
 def test_replay(emu, dims, batch, base, form):
