@@ -473,10 +473,14 @@ int be_device_name(char* buf, int n) {
 }
 
 int be_num_sms() {
+  static std::atomic<int> known[64];  // per device, 0: not asked yet
   int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1)
+  if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+  const bool keep = dev >= 0 && dev < 64;
+  if (keep && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1)
     return 1;
+  if (keep) known[dev].store(n, std::memory_order_relaxed);
   return n;
 }
 

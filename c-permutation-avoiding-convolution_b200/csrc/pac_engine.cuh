@@ -113,6 +113,9 @@ struct PassDesc {
   // lines; null for a plan's own batch
   const long long* poff;
   int logLP;
+  // 1: the tables were complete when the plan was handed out, so a kernel may
+  // read them ahead of the work queued before it
+  int tw_fixed;
   // 1: plane pass of a 3D convolution (pac_plane.cuh): axes 1 and 2 of
   // every plane, whose stages are rlog[0 .. plane_n1s-1] (axis 1) then
   // rlog[plane_n1s .. nst-1] (axis 2), on a cluster of 2^logC CTAs

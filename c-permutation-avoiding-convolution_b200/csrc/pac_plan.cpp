@@ -26,6 +26,7 @@
 #include <stdlib.h>
 #include <stdio.h>
 #include <string.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <map>
@@ -84,6 +85,7 @@ struct Schedule {
   int special = 0;
   int w_shift = 0;
   int plane = 0;        // 3D: 1 plane schedule, -1 line schedule, 0 built-in
+  int tables_fixed = 0; // the tables are complete and stay (allocating plans)
   int whole_tw4 = 1;    // whole 4-step tables for short axes (not for the FP32 forms' FP64
                         // schedule, which only set-up uses)
   int short_cols = 0;   // columns of at most 256 points (batches of problems at any offset)
@@ -102,16 +104,10 @@ struct Schedule {
     std::map<int, void*> tab;
   };
   std::map<int, Tw4> tw4;  // keyed by log N
+  void* block = nullptr;  // the allocation that holds every table
   ~Schedule() {
-    if (pool) be_free(pool);
+    if (block) be_free(block);
     if (tcc) be_free(tcc);
-    for (auto& kv : tw4) {
-      be_free(kv.second.lo);
-      be_free(kv.second.hi);
-      if (kv.second.lo64 != kv.second.lo) be_free(kv.second.lo64);
-      if (kv.second.hi64 != kv.second.hi) be_free(kv.second.hi64);
-      for (auto& t : kv.second.tab) be_free(t.second);
-    }
   }
 };
 
@@ -144,9 +140,7 @@ static int max_factor_log(int bytes, int b2, int cap = 0) {
   return lmax - lmax % b2;
 }
 
-// Device memory for a schedule's tables: cudaMalloc'd (freed by the
-// Schedule), or carved out of caller-supplied scratch (Arena; nothing to
-// free).
+// Device memory for a schedule's tables, carved into 256-byte aligned pieces
 struct Arena {
   char* cur;
   char* end;
@@ -158,11 +152,6 @@ struct Arena {
     return p;
   }
 };
-static int table_alloc(Arena* ar, void** p, size_t bytes) {
-  if (!ar) return be_malloc(p, bytes);
-  *p = ar->take(bytes);
-  return *p ? PAC_SUCCESS : set_error(PAC_ERROR_SIZE, "no-allocation scratch too small");
-}
 
 // Plans with the built-in knobs split every axis for the least time in the
 // passes over 8-byte elements.  The costs are microseconds per 2^24 line-unit
@@ -258,10 +247,16 @@ static int split_axes(Schedule& s, int rank, const int* logs, const int* b2s, in
   return PAC_SUCCESS;
 }
 
-// Stage and 4-step twiddle tables of a split schedule, in memory from
-// table_alloc, generated on `stream`.
-static int build_tables(Schedule& s, Arena* ar, void* stream) {
+// Stage and 4-step twiddle tables of a split schedule, generated on `stream`,
+// in one block: from `ar`, or allocated (s.block, with `extra` zeroed bytes
+// at its start).  One cudaMalloc a schedule: each costs 10 to 100 us.
+static int build_tables(Schedule& s, Arena* ar, void* stream, size_t extra = 0) {
   const int bytes = s.bytes;
+  struct Piece {
+    void** to;
+    size_t bytes;
+  };
+  std::vector<Piece> pieces;
   std::vector<std::pair<int, int>> specs;
   long long total = 0;
   for (size_t i = 0; i < s.vax.size(); ++i) {
@@ -276,54 +271,71 @@ static int build_tables(Schedule& s, Arena* ar, void* stream) {
       logK -= rl;
     }
   }
-  if (total > 0) {
-    PAC_TRY(table_alloc(ar, &s.pool, (size_t)total * 2 * bytes));
-    for (auto& k : specs) {
-      char* dst = (char*)s.pool + (size_t)s.tw_off[k] * 2 * bytes;
-      PAC_TRY(be_fill_stage_tw(dst, bytes, k.first, k.second, stream));
-    }
-  }
+  if (total > 0) pieces.push_back({&s.pool, (size_t)total * 2 * bytes});
   // 4-step twiddles: for every non-last factor, N = L * (later factors of its axis)
   for (size_t i = 0; i < s.vax.size(); ++i) {
     if (s.vax[i].last) continue;
     int logN = 0;
     for (size_t j = i; j < s.vax.size() && s.vax[j].axis == s.vax[i].axis; ++j) logN += s.vax[j].log;
-    if (!ar && !s.tc && s.whole_tw4 && logN <= PAC_TW4_TABLE_LOG) {
-      void*& tab = s.tw4[logN].tab[s.vax[i].log];
-      if (!tab) {
-        PAC_TRY(be_malloc(&tab, (size_t)2 * bytes << logN));
-        PAC_TRY(be_fill_tw4(tab, bytes, s.vax[i].log, logN, stream));
-      }
+    const bool fresh = !s.tw4.count(logN);
+    Schedule::Tw4& t = s.tw4[logN];  // (map nodes stay where they are)
+    if (!ar && !s.tc && s.whole_tw4 && logN <= PAC_TW4_TABLE_LOG && !t.tab.count(s.vax[i].log)) {
+      t.tab[s.vax[i].log] = nullptr;
+      pieces.push_back({&t.tab[s.vax[i].log], (size_t)2 * bytes << logN});
     }
-    if (s.tw4[logN].lo) continue;
-    Schedule::Tw4& t = s.tw4[logN];
+    if (!fresh) continue;
     t.lolog = (logN + 1) / 2;
-    long long nlo = 1LL << t.lolog, nhi = 1LL << (logN - t.lolog);
-    PAC_TRY(table_alloc(ar, &t.lo, (size_t)nlo * 2 * bytes));
-    PAC_TRY(table_alloc(ar, &t.hi, (size_t)nhi * 2 * bytes));
+    const size_t nlo = (size_t)1 << t.lolog, nhi = (size_t)1 << (logN - t.lolog);
+    pieces.push_back({&t.lo, nlo * 2 * bytes});
+    pieces.push_back({&t.hi, nhi * 2 * bytes});
+    if (bytes != 8) {
+      pieces.push_back({&t.lo64, nlo * 16});
+      pieces.push_back({&t.hi64, nhi * 16});
+    }
+  }
+  Arena own{nullptr, nullptr};
+  if (!ar) {
+    size_t need = extra;
+    for (const Piece& p : pieces) need += (p.bytes + 255) & ~(size_t)255;
+    if (need == 0) return PAC_SUCCESS;
+    PAC_TRY(be_malloc(&s.block, need));
+    if (extra) PAC_TRY(be_memset(s.block, 0, extra, stream));
+    own = {(char*)s.block + extra, (char*)s.block + need};
+    ar = &own;
+  }
+  for (const Piece& p : pieces) {
+    *p.to = ar->take(p.bytes);
+    if (!*p.to) return set_error(PAC_ERROR_SIZE, "no-allocation scratch too small");
+  }
+  for (auto& k : specs)
+    PAC_TRY(be_fill_stage_tw((char*)s.pool + (size_t)s.tw_off[k] * 2 * bytes, bytes, k.first,
+                             k.second, stream));
+  for (auto& kv : s.tw4) {
+    const int logN = kv.first;
+    Schedule::Tw4& t = kv.second;
+    const long long nlo = 1LL << t.lolog, nhi = 1LL << (logN - t.lolog);
+    PAC_TRY(be_fill_pow_tw(t.lo, bytes, nlo, 1, logN, stream));
+    PAC_TRY(be_fill_pow_tw(t.hi, bytes, nhi, nlo, logN, stream));
     if (bytes == 8) {
       t.lo64 = t.lo;
       t.hi64 = t.hi;
     } else {
-      PAC_TRY(table_alloc(ar, &t.lo64, (size_t)nlo * 16));
-      PAC_TRY(table_alloc(ar, &t.hi64, (size_t)nhi * 16));
-    }
-    PAC_TRY(be_fill_pow_tw(t.lo, bytes, nlo, 1, logN, stream));
-    PAC_TRY(be_fill_pow_tw(t.hi, bytes, nhi, nlo, logN, stream));
-    if (bytes != 8) {
       PAC_TRY(be_fill_pow_tw(t.lo64, 8, nlo, 1, logN, stream));
       PAC_TRY(be_fill_pow_tw(t.hi64, 8, nhi, nlo, logN, stream));
     }
+    for (auto& f : t.tab) PAC_TRY(be_fill_tw4(f.second, bytes, f.first, logN, stream));
   }
   return PAC_SUCCESS;
 }
 
-static int build_schedule(Schedule& s, int rank, const int* logs, const int* b2s, int bytes) {
+// The tables are filled on the legacy stream, which does not order against
+// non-blocking streams: the caller finishes them before the plan is handed out.
+static int build_schedule(Schedule& s, int rank, const int* logs, const int* b2s, int bytes,
+                          size_t extra = 0) {
   PAC_TRY(split_axes(s, rank, logs, b2s, bytes));
-  PAC_TRY(build_tables(s, nullptr, nullptr));
-  // the tables are filled on the legacy stream, which does not order against
-  // non-blocking streams: finish them before the plan is handed out
-  return be_stream_sync(nullptr);
+  PAC_TRY(build_tables(s, nullptr, nullptr, extra));
+  s.tables_fixed = 1;
+  return PAC_SUCCESS;
 }
 
 }  // namespace pac
@@ -361,7 +373,6 @@ struct pac_plan_s {
   ~pac_plan_s() {
     if (ws) pac::be_free(ws);
     if (tmp64) pac::be_free(tmp64);
-    if (status) pac::be_free(status);
     for (void* e : t_ev) pac::be_event_destroy(e);
   }
 };
@@ -459,16 +470,36 @@ static PassSpec make_pass(const Schedule& s, int vi, long long batch, long long 
   return p;
 }
 
+// The environment's kernel choices, looked up once per call (one getenv per
+// choice and pass took 1 us of a call's 5)
+struct EnvChoice {
+  const char *coltma = nullptr, *pipe = nullptr, *cluster = nullptr, *special = nullptr;
+};
+static EnvChoice env_choice() {
+  EnvChoice c;
+  for (char** e = environ; e && *e; ++e) {
+    const char* v = *e;
+    if (v[0] != 'P' || v[1] != 'A' || v[2] != 'C' || v[3] != '_') continue;
+    auto is = [&](const char* name, const char** to) {
+      const size_t n = strlen(name);
+      if (strncmp(v + 4, name, n) == 0 && v[4 + n] == '=') *to = v + 5 + n;
+    };
+    is("COLTMA", &c.coltma);
+    is("PIPE", &c.pipe);
+    is("CLUSTER_VARIANT", &c.cluster);
+    is("SPECIAL_VARIANT", &c.special);
+  }
+  return c;
+}
+
 // Switch a pass to the kernel over 8-byte elements (pac_vec.cuh) of its
 // geometry.  Plans with knobs and the environment's kernel choices keep the
 // kernels those select, the tensor-core form its own; a column tile has to
 // lie within the stride, and the copies want 16-byte aligned arrays.
-static bool apply_vec(const Schedule& s, PassSpec& p) {
+static bool apply_vec(const Schedule& s, PassSpec& p, const EnvChoice& env) {
   PassDesc& d = p.d;
   if (s.special != 0 || s.w_shift != 0 || s.rlog_cap < 4 || d.tc || d.plane) return false;
-  if (getenv("PAC_COLTMA") || getenv("PAC_PIPE") || getenv("PAC_CLUSTER_VARIANT") ||
-      getenv("PAC_SPECIAL_VARIANT"))
-    return false;
+  if (env.coltma || env.pipe || env.cluster || env.special) return false;
   const int cols = d.logS > 0 ? 1 : 0;
   VecGeo g;
   if (!vec_geometry(p.b2, d.mode, d.sign, d.logL, cols, &g)) return false;
@@ -497,10 +528,10 @@ static bool apply_vec(const Schedule& s, PassSpec& p) {
 
 // Switch a pass to its specialised kernel when pac_special.h has one for its
 // geometry and the tile fits the lines (W divides nlines and the stride).
-static void apply_special(const Schedule& s, PassSpec& p) {
+static void apply_special(const Schedule& s, PassSpec& p, const EnvChoice& env) {
   PassDesc& d = p.d;
   int logW = 0, nt = 0;
-  if (apply_vec(s, p)) return;
+  if (apply_vec(s, p, env)) return;
   if (d.nat || d.plane) return;
   if (s.special < 0) return;  // tuned off
   // column pass whose tile a CTA cluster shares (W columns within the
@@ -508,7 +539,7 @@ static void apply_special(const Schedule& s, PassSpec& p) {
   // candidate geometry of the cluster list
   // (the cluster and pipelined variants have no tensor-core stages)
   // (the cluster and pipelined variants run the radix-16 schedule only)
-  const char* cvar = d.tc || s.rlog_cap < 4 ? nullptr : getenv("PAC_CLUSTER_VARIANT");
+  const char* cvar = d.tc || s.rlog_cap < 4 ? nullptr : env.cluster;
   if (d.logS > 0 && cvar != nullptr) {
     int logC = 0;
     if (cluster_geometry(s.bytes, p.b2, d.mode, d.sign, d.logL, &logW, &logC, &nt, atoi(cvar)) &&
@@ -528,7 +559,7 @@ static void apply_special(const Schedule& s, PassSpec& p) {
   // pipelined column pass, opt-in (PAC_PIPE=1): persistent CTAs, one per
   // SM, tensor-copy prefetch of the next tile (16-byte aligned input arrays
   // for the tensor maps)
-  const char* pipe = d.tc || s.rlog_cap < 4 ? nullptr : getenv("PAC_PIPE");
+  const char* pipe = d.tc || s.rlog_cap < 4 ? nullptr : env.pipe;
   if (d.logS > 0 && cvar == nullptr && pipe != nullptr && atoi(pipe) != 0 &&
       pipe_geometry(s.bytes, p.b2, d.mode, d.sign, d.logL, &logW, &nt) && logW <= d.logS &&
       (d.nlines & ((1LL << logW) - 1)) == 0 && (d.nlines >> d.logS) < (1LL << 31) &&
@@ -550,7 +581,7 @@ static void apply_special(const Schedule& s, PassSpec& p) {
   // candidate of its geometry, 0 none; unset, the geometry's default entry.
   // Plain DIF / DIT passes of the default radix schedule, 16-byte aligned
   // arrays; not with specialised kernels tuned off.
-  const char* tv = getenv("PAC_COLTMA");
+  const char* tv = env.coltma;
   const int tvar = (s.rlog_cap < 4 || s.special < 0) ? 0 : tv ? atoi(tv) : -1;
   int tminb = 1, tpipe = 0, tcand = 0;
   if (d.logS > 0 && cvar == nullptr && tvar != 0 && d.tw4 == 0 &&
@@ -576,7 +607,7 @@ static void apply_special(const Schedule& s, PassSpec& p) {
     if (d.tc) p.smem += (size_t)(nt / 128) * 16384 + 4096;
     return;
   }
-  const char* var = getenv("PAC_SPECIAL_VARIANT");
+  const char* var = env.special;
   int variant = s.special > 0 ? s.special : var ? atoi(var) : 0;
   const int cols = d.logS > 0 ? 1 : 0;
   const int rc = s.rlog_cap < 4 ? s.rlog_cap : 4;
@@ -652,10 +683,12 @@ static int launch(const Schedule& s, PassSpec& p, void* stream, int index = 0) {
 // events and accumulate the per-pass milliseconds in the plan.
 static int exec_passes(pac_plan_s* pl, const Schedule& s, std::vector<PassSpec>& passes,
                        void* stream) {
+  const EnvChoice env = env_choice();
   for (auto& p : passes) {
     p.d.status = pl->status;
     p.d.wait_limit = pl->wait_limit;
-    apply_special(s, p);
+    p.d.tw_fixed = s.tables_fixed;
+    apply_special(s, p, env);
   }
   if (!pl->timing) {
     for (size_t i = 0; i < passes.size(); ++i) PAC_TRY(launch(s, passes[i], stream, (int)i));
@@ -964,6 +997,7 @@ int plan_batch_passes(pac_plan_s* pl, long long copies, const long long* poff, c
                       const void* x_im, const void* h_re, const void* h_im, void* y_re,
                       void* y_im, std::vector<PassDesc>& descs, std::vector<long long>& tiles) {
   const Schedule& s = pl->main;
+  const EnvChoice env = env_choice();
   descs.clear();
   tiles.clear();
   if (s.vax.empty()) return PAC_SUCCESS;
@@ -972,7 +1006,7 @@ int plan_batch_passes(pac_plan_s* pl, long long copies, const long long* poff, c
   int logN = 0;
   for (const VAx& v : s.vax) logN += v.log;
   for (auto& p : passes) {
-    if (!apply_vec(s, p) || (p.d.logS > 0 && p.d.logL > 8)) {
+    if (!apply_vec(s, p, env) || (p.d.logS > 0 && p.d.logL > 8)) {
       descs.clear();
       tiles.clear();
       return PAC_SUCCESS;
@@ -980,6 +1014,7 @@ int plan_batch_passes(pac_plan_s* pl, long long copies, const long long* poff, c
     p.d.poff = poff;
     p.d.logLP = logN - p.d.logL;
     p.d.status = pl->status;
+    p.d.tw_fixed = s.tables_fixed;
     descs.push_back(p.d);
     tiles.push_back(p.grid);
   }
@@ -1055,9 +1090,6 @@ int conv_in_scratch(void* scratch, size_t scratch_bytes, int logn, int batch, co
                        stream);
   if (st == PAC_SUCCESS) st = to_plan_order(&pl, hre, him, 1, hre, him, 1.0, stream);
   if (st == PAC_SUCCESS) st = run_conv(&pl, x_re, x_im, hre, him, 0, y_re, y_im, 1.0, stream);
-  // the tables live in the caller's scratch: nothing to free
-  pl.main.pool = nullptr;
-  pl.main.tw4.clear();
   return st;
 }
 
@@ -1137,7 +1169,9 @@ static int create_plan(pac_plan_t* plan, int rank, const int* dims, const int* d
   p->main.short_cols = short_cols;
   int bytes = form == PAC_FORM_F64 ? 8 : 4;
   p->main.tc = form == PAC_FORM_TC;
-  st = build_schedule(p->main, rank, p->logs, b2s, bytes);
+  // (the status word lies ahead of the tables)
+  st = build_schedule(p->main, rank, p->logs, b2s, bytes, 256);
+  p->status = (int*)p->main.block;
   if (st != PAC_SUCCESS) return st;
   if (p->main.tc) {
     st = be_malloc(&p->main.tcc, sizeof(TcConst) * TC_CONST_SETS * 32);
@@ -1150,9 +1184,7 @@ static int create_plan(pac_plan_t* plan, int rank, const int* dims, const int* d
     st = build_schedule(*p->s64, rank, p->logs, b2s, 8);
     if (st != PAC_SUCCESS) return st;
   }
-  st = be_malloc((void**)&p->status, sizeof(int));
-  if (st == PAC_SUCCESS) st = be_memset(p->status, 0, sizeof(int), nullptr);
-  if (st == PAC_SUCCESS) st = be_stream_sync(nullptr);
+  st = be_stream_sync(nullptr);
   if (st != PAC_SUCCESS) return st;
   *plan = p.release();
   return PAC_SUCCESS;

@@ -117,6 +117,17 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void*
       "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
+// Programmatic dependent launch: the next kernel of the stream may start once
+// every CTA of this one has called pdl_trigger (its CTAs take the place of
+// those that leave); it reads or writes nothing that depends on this kernel
+// before its pdl_wait, which returns when this kernel and all before it are
+// complete.  Both do nothing in a kernel launched without the attribute.
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 __device__ __forceinline__ void bulk_commit() {
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }

@@ -33,6 +33,9 @@ constexpr int kBytes = 4;
 #define PAC_VEC_MINB(M8, M4) M4
 #endif
 
+// shared memory of an SM, and the most that a CTA may ask for (static kept)
+constexpr size_t kSmemSM = 228 * 1024, kSmemCTA = 226 * 1024;
+
 // CTAs that fit the device with this kernel, its shared-memory limit raised
 // (once per kernel and device)
 struct Resident {
@@ -49,7 +52,7 @@ int resident(Resident& r, K kern, int nt, size_t smem, long long* out) {
     *out = r.ctas[dev];
     return PAC_SUCCESS;
   }
-  PAC_CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+  PAC_CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCTA),
          "cudaFuncSetAttribute");
   int nb = 0, sms = 0;
   PAC_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, nt, smem),
@@ -59,6 +62,40 @@ int resident(Resident& r, K kern, int nt, size_t smem, long long* out) {
   if (nb < 1) return set_error(PAC_ERROR_INTERNAL, "pass over 8-byte elements does not fit an SM");
   if (keep) r.ctas[dev] = nb * sms;
   *out = (long long)nb * sms;
+  return PAC_SUCCESS;
+}
+
+// A launch that may overlap the end of the work before it in the stream: the
+// kernels set up (barriers, twiddles in shared memory) and then wait for that
+// work (pdl_wait).  slots: CTAs that fit the device (negative: a CTA a tile,
+// else persistent CTAs; 0 unknown).  Fewer tiles than that have to be spread
+// over the SMs: CTAs that arrive while the kernel before still runs would
+// otherwise pile up on the SMs that it leaves first, so each reserves its
+// share of an SM's shared memory.
+template <class K, class... A>
+int pdl_launch(K kern, long long tiles, long long slots, int nt, size_t smem, cudaStream_t st,
+               const A&... args) {
+  const long long fit = slots < 0 ? -slots : slots;
+  long long grid = tiles;
+  if (slots > 0 && tiles > slots) grid = slots;
+  if (fit > 0 && tiles < fit) {
+    const int sms = be_num_sms();
+    const long long per_sm = (tiles + sms - 1) / sms;
+    const size_t share = (size_t)(kSmemSM / per_sm) / 1024 * 1024 - 2048;
+    if (share > smem) smem = share < kSmemCTA ? share : kSmemCTA;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)nt);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  PAC_CU(cudaLaunchKernelEx(&cfg, kern, args...), "pass over 8-byte elements");
+  count_launch();
   return PAC_SUCCESS;
 }
 
@@ -88,10 +125,7 @@ int rows_as(const PassDesc& d, cudaStream_t st) {
   int s = resident(res, kern, NT, VP::SMEM + 128, &slots);
   if (s != PAC_SUCCESS || d.vec == VEC_PREPARE) return s;
   const long long wl = VP::W * VP::LPU, tiles = (d.nlines + wl - 1) / wl;
-  kern<<<(unsigned)(tiles < slots ? tiles : slots), NT, VP::SMEM + 128, st>>>(d);
-  PAC_CU(cudaGetLastError(), "pac_vec_rows_kernel launch");
-  count_launch();
-  return PAC_SUCCESS;
+  return pdl_launch(kern, tiles, slots, NT, VP::SMEM + 128, st, d);
 }
 
 // column tiles read straight from global memory
@@ -105,10 +139,7 @@ int cols_direct(const PassDesc& d, cudaStream_t st) {
   if (s != PAC_SUCCESS || d.vec == VEC_PREPARE) return s;
   const long long tiles = (d.nlines / VP::LPU) >> LOGW;
   if (tiles > 0x7fffffffLL) return set_error(PAC_ERROR_SIZE, "pass grid too large");
-  kern<<<(unsigned)tiles, NT, VP::TILE_BYTES, st>>>(d);
-  PAC_CU(cudaGetLastError(), "pac_vec_direct_kernel launch");
-  count_launch();
-  return PAC_SUCCESS;
+  return pdl_launch(kern, tiles, -slots, NT, VP::TILE_BYTES, st, d);
 }
 
 // column tiles brought in by tensor copies, 16 elements a thread
@@ -125,10 +156,15 @@ int cols_copied(const PassDesc& d, cudaStream_t st) {
   if ((s = col_map<VP>(&m[0], d.in_re, d)) != PAC_SUCCESS) return s;
   if ((s = col_map<VP>(&m[1], d.in_im, d)) != PAC_SUCCESS) return s;
   const long long tiles = (d.nlines / VP::LPU) >> LOGW;
-  kern<<<(unsigned)(tiles < slots ? tiles : slots), T, VP::SMEM + 128, st>>>(d, m[0], m[1]);
-  PAC_CU(cudaGetLastError(), "pac_vec_cols_kernel launch");
-  count_launch();
-  return PAC_SUCCESS;
+  if (tiles > 4 * slots) {
+    // rounds enough to hide a launch; as a dependent launch these wide CTAs
+    // cost 512 x 256 x 128 FP64 1.2%
+    kern<<<(unsigned)slots, T, VP::SMEM + 128, st>>>(d, m[0], m[1]);
+    PAC_CU(cudaGetLastError(), "pac_vec_cols_kernel launch");
+    count_launch();
+    return PAC_SUCCESS;
+  }
+  return pdl_launch(kern, tiles, slots, T, VP::SMEM + 128, st, d, m[0], m[1]);
 }
 
 template <int B2, int MODE, int SIGN, int LOGL, int TW4, int OFFS>
@@ -141,10 +177,7 @@ int small_as(const PassDesc& d, cudaStream_t st) {
     PAC_CU(cudaFuncGetAttributes(&fa, kern), "cudaFuncGetAttributes");
     return PAC_SUCCESS;
   }
-  kern<<<(unsigned)grid, 256, 0, st>>>(d);
-  PAC_CU(cudaGetLastError(), "pac_vec_small_kernel launch");
-  count_launch();
-  return PAC_SUCCESS;
+  return pdl_launch(kern, grid, 0, 256, 0, st, d);
 }
 
 // problems at any offset: convolutions only

@@ -958,7 +958,7 @@ struct VecPass {
         if constexpr (S == 0 && DIRECT) read_g(d, tile, t, x);
         else read<S, S == 0 && !RELAY_IN>(t, B, x);
       });
-      if constexpr (!DIRECT && S == STEPS - 1 && !RELAY_OUT) ex.freed();
+      if constexpr (S == STEPS - 1 && !RELAY_OUT) ex.freed();
       if constexpr (CONV && S == NS - 1) {
         ex.each_mid([&](int t, CV<V>(&x)[TPT], auto& m) { middle(d, tile, t, m, x); });
       } else {

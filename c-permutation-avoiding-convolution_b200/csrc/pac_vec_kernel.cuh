@@ -51,7 +51,8 @@ struct VecExec {
   __device__ __forceinline__ void freed() {
     fence_proxy_async();
     sync();
-    if (threadIdx.x == 0 && next < ntiles) issue(next);
+    if (next >= ntiles) pdl_trigger();
+    else if (threadIdx.x == 0) issue(next);
   }
 };
 
@@ -64,12 +65,14 @@ __device__ __forceinline__ void vec_tiles(const PassDesc& d, CV<V>* B, uint64_t*
     mbar_init(bar, 1);
     fence_barrier_init();
   }
+  using Real = typename VP::Real;
+  Cx<Real>* tws = reinterpret_cast<Cx<Real>*>(B + VP::TILE);
+  if (!d.tw_fixed) pdl_wait();
+  VP::tw_fill(d, threadIdx.x, tws);  // read after the first tile's barrier
+  if (d.tw_fixed) pdl_wait();
   __syncthreads();
   long long tile = blockIdx.x;
   if (threadIdx.x == 0 && tile < ntiles) issue(tile);
-  using Real = typename VP::Real;
-  Cx<Real>* tws = reinterpret_cast<Cx<Real>*>(B + VP::TILE);
-  VP::tw_fill(d, threadIdx.x, tws);  // read after the first tile's barrier
   uint32_t phase = 0;
   VecExec<VP, V, Issue> ex{{}, {}, tile, ntiles, issue};
   for (; tile < ntiles; tile += gridDim.x) {
@@ -160,7 +163,7 @@ struct VecExecOnce {
     f((int)threadIdx.x, x);
   }
   __device__ __forceinline__ void sync() { vec_sync<VP::kThreads>(); }
-  __device__ __forceinline__ void freed() {}
+  __device__ __forceinline__ void freed() { pdl_trigger(); }
 };
 template <class V, int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int MINB, int TW4,
           int OFFS>
@@ -170,12 +173,15 @@ __global__ void __launch_bounds__(NT, MINB) pac_vec_direct_kernel(const __grid_c
   extern __shared__ __align__(16) unsigned char pac_smem_raw[];
   CV<V>* B = reinterpret_cast<CV<V>*>(pac_smem_raw);
   VecExecOnce<VP, V> ex;
+  pdl_wait();
   VP::template body<TW4>(d, blockIdx.x, B, (const Cx<Real>*)nullptr, ex);
 }
 
 template <class V, int B2, int MODE, int SIGN, int LOGL, int TW4, int OFFS>
 __global__ void __launch_bounds__(256) pac_vec_small_kernel(const __grid_constant__ PassDesc d) {
   const long long u = (long long)blockIdx.x * 256 + threadIdx.x;
+  pdl_wait();
+  pdl_trigger();
   if (u < d.nlines / VT<V>::LPU) VecSmall<V, B2, MODE, SIGN, LOGL, OFFS>::template run<TW4>(d, u);
 }
 

@@ -87,3 +87,44 @@ def test_replay(emu, dims, batch, base, form):
 @pytest.mark.parametrize("dims,batch,base", ROWS + COLS + SPLIT + LONG)
 def test_gpu(lib, dims, batch, base, form):
     check(lib, dims, batch, base, form)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", [F64, F32])
+@pytest.mark.parametrize("dims,batch,base", [((4096,), 3, 2), ((256, 256), 1, 2), ((1 << 16,), 5, 2),
+                                             ((1024, 512), 2, 2), ((64, 64, 64), 1, 4)])
+def test_queued_calls(lib, dims, batch, base, form):
+    """Calls queued on one stream that each overwrite their own input (every
+    kernel may start before the one ahead of it has ended) give bit for bit
+    what the same calls give when each is waited for."""
+    dt = np.float64 if form == F64 else np.float32
+    g = rng(5)
+    shape = (batch,) + dims
+    n = int(np.prod(dims))
+    h = np.zeros(dims)
+    h[(0,) * len(dims)] = 0.9
+    h[(1,) * len(dims)] = 0.3
+    d = P.Dev(lib)
+    got = []
+    try:
+        plan = pac.Plan(lib, dims, batch, base, form)
+        hr, hi = d.put(h), d.put(0.5 * h)
+        Hr, Hi = d.zeros(dims, dt), d.zeros(dims, dt)
+        plan.filter_spectrum(hr, hi, Hr, Hi)
+        x = [g.standard_normal(shape).astype(dt) for _ in range(2)]
+        for wait in (True, False):
+            xr, xi = d.put(x[0]), d.put(x[1])
+            for k in range(24):
+                if k % 3 == 2:
+                    plan.transform(pac.OP_FFT, xr, xi, xr, xi)
+                    plan.transform(pac.OP_IFFT, xr, xi, xr, xi)
+                else:
+                    plan.convolve(xr, xi, Hr, Hi, xr, xi)
+                if wait:
+                    pac.check(lib, lib.pac_stream_synchronize(None), "sync")
+            got.append((d.get(xr, shape, dt), d.get(xi, shape, dt)))
+        plan.close()
+    finally:
+        d.free()
+    assert n and np.isfinite(got[0][0]).all()
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
