@@ -172,12 +172,17 @@ static bool builtin_split(const Schedule& s) {
 // the cheapest split of an axis of 2^lg, digit base 2^b2, into at most three
 // factors; rows: its last factor is the innermost of the plan.  Empty when
 // some factor would have no kernel (short axes, long axes of large bases).
-static std::vector<int> cheapest_split(int lg, int b2, bool rows, bool short_cols) {
+static std::vector<int> cheapest_split(int lg, int b2, bool rows, bool short_cols,
+                                       long long lines) {
   std::vector<int> best, cur;
   int best_cost = 1 << 30;
   VecGeo g;
   auto cost = [&](int f, bool last) {
     const bool row = rows && last;
+    // one CTA takes 15 us for an 8192-point line: fewer lines than keep half
+    // the SMs busy are faster in three passes of many tiles (one line 15 us
+    // against 9.5)
+    if (row && f == 13 && lines < 64) return 0;
     if (f > 13 || (short_cols && !row && f > 8) || !vec_geometry(b2, row ? MODE_CONV : MODE_DIF, -1, f, row ? 0 : 1, &g)) return 0;
     return row ? kCostRow[f] : 2 * (last ? kCostCol[f] : kCostTw4[f]);
   };
@@ -208,15 +213,20 @@ static std::vector<int> cheapest_split(int lg, int b2, bool rows, bool short_col
 
 // The factors of every axis and their stage radices -- the one rule every
 // plan follows (allocating plans and the no-allocation entry point alike).
-static int split_axes(Schedule& s, int rank, const int* logs, const int* b2s, int bytes) {
+static int split_axes(Schedule& s, int rank, const int* logs, const int* b2s, int bytes,
+                      long long batch) {
   s.bytes = bytes;
+  // lines of the last axis (pairs of them in FP32)
+  long long lines = batch;
+  for (int a = 0; a + 1 < rank; ++a) lines <<= logs[a];
+  lines = bytes == 8 ? lines : (lines + 1) / 2;
   s.b2 = b2s[rank - 1];
   for (int a = 0; a < rank; ++a) {
     int lg = logs[a];
     if (lg == 0) continue;
     const int b2 = b2s[a];
     if (builtin_split(s)) {
-      const std::vector<int> f = cheapest_split(lg, b2, a == rank - 1, s.short_cols);
+      const std::vector<int> f = cheapest_split(lg, b2, a == rank - 1, s.short_cols, lines);
       for (size_t i = 0; i < f.size(); ++i)
         s.vax.push_back({f[i], a, i == 0, i + 1 == f.size(), b2});
       if (!f.empty()) continue;
@@ -331,8 +341,8 @@ static int build_tables(Schedule& s, Arena* ar, void* stream, size_t extra = 0) 
 // The tables are filled on the legacy stream, which does not order against
 // non-blocking streams: the caller finishes them before the plan is handed out.
 static int build_schedule(Schedule& s, int rank, const int* logs, const int* b2s, int bytes,
-                          size_t extra = 0) {
-  PAC_TRY(split_axes(s, rank, logs, b2s, bytes));
+                          long long batch, size_t extra = 0) {
+  PAC_TRY(split_axes(s, rank, logs, b2s, bytes, batch));
   PAC_TRY(build_tables(s, nullptr, nullptr, extra));
   s.tables_fixed = 1;
   return PAC_SUCCESS;
@@ -1062,9 +1072,9 @@ static int to_plan_order(pac_plan_s* pl, const double* in_re, const double* in_i
 // call never depends on what an earlier call left there.  Nothing here
 // allocates device memory.
 // ---------------------------------------------------------------------------
-static int build_schedule_in_arena(Schedule& s, int logn, Arena& ar, void* stream) {
+static int build_schedule_in_arena(Schedule& s, int logn, int batch, Arena& ar, void* stream) {
   const int logs[1] = {logn}, b2s[1] = {1};
-  if (logn > 0) PAC_TRY(split_axes(s, 1, logs, b2s, 8));
+  if (logn > 0) PAC_TRY(split_axes(s, 1, logs, b2s, 8, batch));
   return build_tables(s, &ar, stream);
 }
 
@@ -1080,7 +1090,7 @@ int conv_in_scratch(void* scratch, size_t scratch_bytes, int logn, int batch, co
   pl.form = PAC_FORM_F64;
   pl.N = 1LL << logn;
   Arena ar{(char*)scratch, (char*)scratch + scratch_bytes};
-  int st = build_schedule_in_arena(pl.main, logn, ar, stream);
+  int st = build_schedule_in_arena(pl.main, logn, batch, ar, stream);
   double* hre = (double*)ar.take((size_t)pl.N * 8);
   double* him = (double*)ar.take((size_t)pl.N * 8);
   if (st == PAC_SUCCESS && (!hre || !him))
@@ -1170,7 +1180,7 @@ static int create_plan(pac_plan_t* plan, int rank, const int* dims, const int* d
   int bytes = form == PAC_FORM_F64 ? 8 : 4;
   p->main.tc = form == PAC_FORM_TC;
   // (the status word lies ahead of the tables)
-  st = build_schedule(p->main, rank, p->logs, b2s, bytes, 256);
+  st = build_schedule(p->main, rank, p->logs, b2s, bytes, batch, 256);
   p->status = (int*)p->main.block;
   if (st != PAC_SUCCESS) return st;
   if (p->main.tc) {
@@ -1181,7 +1191,7 @@ static int create_plan(pac_plan_t* plan, int rank, const int* dims, const int* d
   if (bytes != 8) {
     p->s64.reset(new Schedule());
     p->s64->whole_tw4 = 0;
-    st = build_schedule(*p->s64, rank, p->logs, b2s, 8);
+    st = build_schedule(*p->s64, rank, p->logs, b2s, 8, batch);
     if (st != PAC_SUCCESS) return st;
   }
   st = be_stream_sync(nullptr);

@@ -14,9 +14,10 @@ from conftest import pac, rng
 
 F64, F32 = pac.PAC_FORM_F64, pac.PAC_FORM_F32
 
-# rows of every length and base (dims, batch, base)
+# rows of every length and base (dims, batch, base); 8192-point rows are one
+# pass from 64 line units on
 ROWS = ([((1 << k,), b, 2) for k in range(5, 14) for b in (1, 3)] +
-        [((64,), 67, 2), ((256,), 9, 2), ((512,), 2, 2), ((1024,), 5, 2)] +
+        [((8192,), 131, 2), ((64,), 67, 2), ((256,), 9, 2), ((512,), 2, 2), ((1024,), 5, 2)] +
         [((4 ** k,), 5, 4) for k in range(3, 7)] + [((8 ** k,), 5, 8) for k in range(2, 5)])
 # columns of every length and base: at the narrowest stride that has a tile
 # of both types, and one with several tiles
