@@ -53,9 +53,9 @@ void nan_fill(std::vector<CV<V>>& b) {
   }
 }
 
-template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int OFFS>
+template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int OFFS, int PORD = 0>
 int rows_as(const PassDesc& d) {
-  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 0, LOGW, NT, 0, OFFS>;
+  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 0, LOGW, NT, 0, OFFS, PORD>;
   using Real = typename VP::Real;
   std::vector<CV<V>> buf((size_t)VP::TILE);
   V* D = (V*)buf.data();
@@ -131,6 +131,10 @@ int no_offsets() {
 }
 template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT>
 int go_rows(const PassDesc& d) {
+  if constexpr (kBytes == 8 && MODE == MODE_DIF && SIGN < 0) {
+    if (d.porder == 8) return rows_as<B2, MODE, SIGN, LOGL, LOGW, NT, 0, 8>(d);
+    if (d.porder == 4) return rows_as<B2, MODE, SIGN, LOGL, LOGW, NT, 0, 4>(d);
+  }
   if (!d.poff) return rows_as<B2, MODE, SIGN, LOGL, LOGW, NT, 0>(d);
   if constexpr (MODE == MODE_CONV) return rows_as<B2, MODE, SIGN, LOGL, LOGW, NT, 1>(d);
   else return no_offsets();

@@ -113,6 +113,10 @@ struct PassDesc {
   // lines; null for a plan's own batch
   const long long* poff;
   int logLP;
+  // filter spectrum: this DIF pass over FP64 rows stores plan order (blocks of
+  // 2^porder_logR positions transposed) in elements of porder bytes; 0: no
+  int porder;
+  int porder_logR;
   // 1: the tables were complete when the plan was handed out, so a kernel may
   // read them ahead of the work queued before it
   int tw_fixed;

@@ -214,14 +214,15 @@ static std::vector<int> cheapest_split(int lg, int b2, bool rows, bool short_col
 // The factors of every axis and their stage radices -- the one rule every
 // plan follows (allocating plans and the no-allocation entry point alike).
 static int split_axes(Schedule& s, int rank, const int* logs, const int* b2s, int bytes,
-                      long long batch) {
+                      long long batch, const Schedule* like = nullptr) {
   s.bytes = bytes;
   // lines of the last axis (pairs of them in FP32)
   long long lines = batch;
   for (int a = 0; a + 1 < rank; ++a) lines <<= logs[a];
   lines = bytes == 8 ? lines : (lines + 1) / 2;
   s.b2 = b2s[rank - 1];
-  for (int a = 0; a < rank; ++a) {
+  if (like) s.vax = like->vax;
+  for (int a = 0; a < rank && !like; ++a) {
     int lg = logs[a];
     if (lg == 0) continue;
     const int b2 = b2s[a];
@@ -341,8 +342,8 @@ static int build_tables(Schedule& s, Arena* ar, void* stream, size_t extra = 0) 
 // The tables are filled on the legacy stream, which does not order against
 // non-blocking streams: the caller finishes them before the plan is handed out.
 static int build_schedule(Schedule& s, int rank, const int* logs, const int* b2s, int bytes,
-                          long long batch, size_t extra = 0) {
-  PAC_TRY(split_axes(s, rank, logs, b2s, bytes, batch));
+                          long long batch, size_t extra = 0, const Schedule* like = nullptr) {
+  PAC_TRY(split_axes(s, rank, logs, b2s, bytes, batch, like));
   PAC_TRY(build_tables(s, nullptr, nullptr, extra));
   s.tables_fixed = 1;
   return PAC_SUCCESS;
@@ -967,6 +968,43 @@ static void build_conv_passes(pac_plan_s* pl, const void* x_re, const void* x_im
   }
 }
 
+// The filter spectrum straight in plan order and storage type: A^T h by the
+// FP64 schedule s, whose last pass stores it so (tmp: FP64 arrays of nfilters
+// problems for the passes before it, may be hhat in FP64).  *done = 0 and
+// nothing launched where that pass has no such kernel (pac_vec.cuh) or the
+// plan's lines differ from s's.
+static bool spectrum_direct(pac_plan_s* pl, const Schedule& s) {
+  return s.bytes == 8 && !s.vax.empty() && !pl->main.vax.empty() &&
+         s.vax.back().log == pl->main.vax.back().log && s.vax.back().b2 == pl->main.vax.back().b2;
+}
+static int run_spectrum(pac_plan_s* pl, const Schedule& s, long long nfilters, const double* h_re,
+                        const double* h_im, void* hhat_re, void* hhat_im, double* tmp_re,
+                        double* tmp_im, double scale, void* stream, int* done) {
+  *done = 0;
+  const int m = (int)s.vax.size();
+  std::vector<PassSpec> passes;
+  for (int vi = 0; vi < m; ++vi) {
+    PassSpec p = make_pass(s, vi, nfilters, pl->N);
+    p.d.mode = MODE_DIF;
+    p.d.sign = -1;
+    p.d.tw4 = s.vax[vi].last ? 0 : 1;
+    p.d.in_re = vi == 0 ? h_re : tmp_re;
+    p.d.in_im = vi == 0 ? h_im : tmp_im;
+    p.d.out_re = vi == m - 1 ? hhat_re : tmp_re;
+    p.d.out_im = vi == m - 1 ? hhat_im : tmp_im;
+    passes.push_back(p);
+  }
+  PassDesc& d = passes.back().d;
+  d.use_scale = 1;
+  d.scale = scale;
+  d.porder_logR = pl->main.rad.back().back();
+  PassSpec probe = passes.back();
+  if (!apply_vec(s, probe, env_choice())) return PAC_SUCCESS;
+  d.porder = pl->main.bytes;
+  *done = 1;
+  return exec_passes(pl, s, passes, stream);
+}
+
 static int run_conv(pac_plan_s* pl, const void* x_re, const void* x_im, const void* h_re,
                     const void* h_im, int per_problem, void* y_re, void* y_im, double scale,
                     void* stream) {
@@ -1191,7 +1229,9 @@ static int create_plan(pac_plan_t* plan, int rank, const int* dims, const int* d
   if (bytes != 8) {
     p->s64.reset(new Schedule());
     p->s64->whole_tw4 = 0;
-    st = build_schedule(*p->s64, rank, p->logs, b2s, 8, batch);
+    // (the same factors, so that the spectrum's last pass can store plan order)
+    st = build_schedule(*p->s64, rank, p->logs, b2s, 8, batch, 0,
+                        builtin_split(p->main) ? &p->main : nullptr);
     if (st != PAC_SUCCESS) return st;
   }
   st = be_stream_sync(nullptr);
@@ -1267,14 +1307,33 @@ PAC_API int pac_filter_spectrum(pac_plan_t plan, const double* h_re, const doubl
   if (nfilters != 1 && nfilters != plan->batch)
     return set_error(PAC_ERROR_INVALID_VALUE, "pac_filter_spectrum: nfilters must be 1 or batch");
   if (plan->form == PAC_FORM_F64) {
+    if (spectrum_direct(plan, plan->main)) {
+      int done = 0;
+      PAC_TRY(run_spectrum(plan, plan->main, nfilters, h_re, h_im, hhat_re, hhat_im,
+                           (double*)hhat_re, (double*)hhat_im, scale, stream, &done));
+      if (done) return PAC_SUCCESS;
+    }
     // A^T h in P order straight into hhat, then reordered in place
     PAC_TRY(run_transform(plan, plan->main, PAC_OP_AT, nfilters, h_re, h_im, hhat_re, hhat_im,
                           scale, 1, stream));
     return to_plan_order(plan, (const double*)hhat_re, (const double*)hhat_im, nfilters, hhat_re,
                          hhat_im, 1.0, stream);
   }
-  // F32 form: FP64 transform into a temporary, reordered and rounded once
+  // F32 form: FP64 transform, reordered and rounded once
   std::lock_guard<std::mutex> g(plan->ws_mu);
+  const bool direct = spectrum_direct(plan, *plan->s64);
+  // (one pass reads h while it writes hhat: not where they share memory)
+  const size_t hb = (size_t)nfilters * plan->N;
+  auto apart = [&](const double* a, void* b) {
+    return (char*)b >= (char*)(a + hb) || (char*)a >= (char*)b + hb * sizeof(float);
+  };
+  if (direct && plan->s64->vax.size() == 1 && apart(h_re, hhat_re) && apart(h_re, hhat_im) &&
+      apart(h_im, hhat_re) && apart(h_im, hhat_im)) {
+    int done = 0;
+    PAC_TRY(run_spectrum(plan, *plan->s64, nfilters, h_re, h_im, hhat_re, hhat_im, nullptr,
+                         nullptr, scale, stream, &done));
+    if (done) return PAC_SUCCESS;
+  }
   size_t need = (size_t)nfilters * plan->N * 2 * sizeof(double);
   if (plan->tmp64_bytes < need) {
     if (plan->tmp64) be_free(plan->tmp64);
@@ -1285,6 +1344,12 @@ PAC_API int pac_filter_spectrum(pac_plan_t plan, const double* h_re, const doubl
   }
   double* tre = (double*)plan->tmp64;
   double* tim = tre + (size_t)nfilters * plan->N;
+  if (direct) {
+    int done = 0;
+    PAC_TRY(run_spectrum(plan, *plan->s64, nfilters, h_re, h_im, hhat_re, hhat_im, tre, tim, scale,
+                         stream, &done));
+    if (done) return PAC_SUCCESS;
+  }
   // the FP64 schedule never needs the workspace for A^T
   PAC_TRY(run_transform(plan, *plan->s64, PAC_OP_AT, nfilters, h_re, h_im, tre, tim, scale, 1,
                         stream));

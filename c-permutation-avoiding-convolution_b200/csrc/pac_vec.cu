@@ -116,11 +116,11 @@ int col_map(CUtensorMap* m, const void* base, const PassDesc& d) {
   return PAC_SUCCESS;
 }
 
-template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int MINB, int OFFS>
+template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int MINB, int OFFS, int PORD = 0>
 int rows_as(const PassDesc& d, cudaStream_t st) {
-  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 0, LOGW, NT, 0, OFFS>;
+  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 0, LOGW, NT, 0, OFFS, PORD>;
   static Resident res;
-  auto kern = pac_vec_rows_kernel<V, B2, MODE, SIGN, LOGL, LOGW, NT, MINB, OFFS>;
+  auto kern = pac_vec_rows_kernel<V, B2, MODE, SIGN, LOGL, LOGW, NT, MINB, OFFS, PORD>;
   long long slots = 0;
   int s = resident(res, kern, NT, VP::SMEM + 128, &slots);
   if (s != PAC_SUCCESS || d.vec == VEC_PREPARE) return s;
@@ -190,6 +190,10 @@ int no_offsets() {
 
 template <int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int MINB>
 int go_rows(const PassDesc& d, cudaStream_t st) {
+  if constexpr (kBytes == 8 && MODE == MODE_DIF && SIGN < 0) {
+    if (d.porder == 8) return rows_as<B2, MODE, SIGN, LOGL, LOGW, NT, MINB, 0, 8>(d, st);
+    if (d.porder == 4) return rows_as<B2, MODE, SIGN, LOGL, LOGW, NT, MINB, 0, 4>(d, st);
+  }
   if (!d.poff) return rows_as<B2, MODE, SIGN, LOGL, LOGW, NT, MINB, 0>(d, st);
   if constexpr (MODE == MODE_CONV) return rows_as<B2, MODE, SIGN, LOGL, LOGW, NT, MINB, 1>(d, st);
   else return no_offsets();

@@ -477,7 +477,7 @@ PAC_HD long long unit_base(const PassDesc& d, long long u) {
 // The pass
 // ---------------------------------------------------------------------------
 template <class V, int B2, int MODE, int SIGN, int LOGL, int COLS, int LOGW, int NT, int DIR = 0,
-          int OFFS = 0>
+          int OFFS = 0, int PORD = 0>
 struct VecPass {
   using Real = typename VT<V>::Real;
   using RS = RadsFor<LOGL, B2>;
@@ -929,14 +929,31 @@ struct VecPass {
     });
   }
   // DIF rows: out of the buffer, consecutive elements of a line by
-  // consecutive threads, in digit-reversed (the slots) or natural order
+  // consecutive threads, in digit-reversed (the slots), natural or plan order
+  // (a filter spectrum: the pass after the transform that reordered and
+  // rounded it is gone)
   static PAC_HD void relay_store(const PassDesc& d, long long tile, int t, const CV<V>* B) {
     const V sc = VT<V>::set(d.scale);
     static_for<TPT>([&](auto kk) {
       const int q = t + kk.value * NT;
       const int w = q >> LOGL, e = q & (L - 1);
-      CV<V> v = vget(B + phys(w, d.nat ? (int)drev<B2>((uint32_t)e, LOGL) : e));
+      int slot = e;
+      if constexpr (PORD != 0) {
+        const int lq = LOGL - d.porder_logR;
+        slot = ((e & ((1 << lq) - 1)) << d.porder_logR) + (e >> lq);
+      } else if (d.nat) {
+        slot = (int)drev<B2>((uint32_t)e, LOGL);
+      }
+      CV<V> v = vget(B + phys(w, slot));
       if (d.use_scale) v = {vmul(v.re, sc), vmul(v.im, sc)};
+      if constexpr (PORD == 4) {  // FP64 lines, rounded once
+        const long long l = (tile << LOGW) + w;
+        if (l < d.nlines) {
+          ((float*)d.out_re)[(l << LOGL) + e] = (float)v.re;
+          ((float*)d.out_im)[(l << LOGL) + e] = (float)v.im;
+        }
+        return;
+      }
       put_row(row_out(d, tile, w, e), 0, v);
     });
   }

@@ -93,9 +93,9 @@ __device__ __forceinline__ void vec_tiles(const PassDesc& d, CV<V>* B, uint64_t*
 }
 
 template <class V, int B2, int MODE, int SIGN, int LOGL, int LOGW, int NT, int MINB,
-          int OFFS>
+          int OFFS, int PORD>
 __global__ void __launch_bounds__(NT, MINB) pac_vec_rows_kernel(const __grid_constant__ PassDesc d) {
-  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 0, LOGW, NT, 0, OFFS>;
+  using VP = VecPass<V, B2, MODE, SIGN, LOGL, 0, LOGW, NT, 0, OFFS, PORD>;
   using Real = typename VP::Real;
   extern __shared__ unsigned char pac_smem_raw[];
   __shared__ __align__(8) uint64_t bar;

@@ -129,3 +129,54 @@ def test_queued_calls(lib, dims, batch, base, form):
         d.free()
     assert n and np.isfinite(got[0][0]).all()
     assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
+# filter spectra stored in plan order by the transform's last pass: every row
+# length, several filters, and a plan whose main schedule has other lines (the
+# reorder stays a pass of its own); FP32 with h and hhat in the same memory
+SPECTRA = ([((1 << k,), 3, 2, None) for k in (5, 6, 7, 8, 9, 10, 11, 12)] +
+           [((8192,), 65, 2, None), ((1 << 15,), 2, 2, None), ((32, 512), 1, 2, None),
+            ((4 ** 5,), 2, 4, None), ((8 ** 3,), 3, 8, None),
+            ((1 << 14,), 2, 2, {"max_factor_log": 5}), ((1024,), 2, 2, {"max_radix_log": 3})])
+
+
+def check_spectrum(L, dims, nf, base, tune, form):
+    dt = np.float64 if form == F64 else np.float32
+    shape = (nf,) + dims
+    g = rng(3)
+    h = [g.standard_normal(shape) for _ in range(2)]
+    d = P.Dev(L)
+    try:
+        plan = pac.Plan(L, dims, nf, base, form, tune=tune)
+        want = [d.zeros(shape, dt) for _ in range(2)]
+        p64 = pac.Plan(L, dims, nf, base, F64)
+        hp, at = [d.put(v) for v in h], [d.zeros(shape, np.float64) for _ in range(2)]
+        p64.transform(pac.OP_AT, *hp, *at)
+        pac.check(L, L.pac_spectrum_to_plan_order(plan.h, *at, nf, *want, 0.25, None), "order")
+        want = [d.get(p, shape, dt) for p in want]
+        got = []
+        for alias in (False, True):  # hhat apart from h, and on top of it
+            hp = [d.put(v) for v in h]
+            out = hp if alias else [d.zeros(shape, dt) for _ in range(2)]
+            plan.filter_spectrum(*hp, *out, nfilters=nf, scale=0.25)
+            got.append([d.get(p, shape, dt) for p in out])
+        plan.close()
+        p64.close()
+    finally:
+        d.free()
+    z = want[0] + 1j * want[1]
+    for a in got:
+        assert P.crel(a[0] + 1j * a[1], z) < (P.TOL if form == F64 else P.TOL_F32)
+
+
+@pytest.mark.parametrize("form", [F64, F32])
+@pytest.mark.parametrize("dims,nf,base,tune", SPECTRA)
+def test_spectrum_replay(emu, dims, nf, base, tune, form):
+    check_spectrum(emu, dims, nf, base, tune, form)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", [F64, F32])
+@pytest.mark.parametrize("dims,nf,base,tune", SPECTRA)
+def test_spectrum_gpu(lib, dims, nf, base, tune, form):
+    check_spectrum(lib, dims, nf, base, tune, form)
