@@ -19,6 +19,12 @@ int be_num_sms();  // streaming multiprocessors of the current device (>= 1)
 int be_device_name(char* buf, int n);  // the current device's name (tuning cache key)
 int be_malloc(void** p, size_t bytes);
 int be_free(void* p);
+int be_host_alloc(void** p, size_t bytes);  // pinned host memory
+int be_host_free(void* p);
+int be_get_device();
+void be_set_device(int device);
+int be_sync_event_create(void** ev);  // no timing, its waiter sleeps
+int be_event_wait(void* ev);
 int be_memcpy(void* dst, const void* src, size_t bytes, int kind, void* stream);
 int be_memset(void* dst, int value, size_t bytes, void* stream);
 int be_stream_create(void** s);

@@ -498,6 +498,34 @@ int be_free(void* p) {
   return PAC_SUCCESS;
 }
 
+int be_host_alloc(void** p, size_t bytes) {
+  cudaError_t e = cudaHostAlloc(p, bytes ? bytes : 16, cudaHostAllocPortable);
+  if (e != cudaSuccess) {
+    *p = nullptr;
+    return set_error(PAC_ERROR_ALLOC, "cudaHostAlloc(%zu): %s", bytes, cudaGetErrorString(e));
+  }
+  return PAC_SUCCESS;
+}
+int be_host_free(void* p) {
+  if (p) PAC_CU(cudaFreeHost(p), "cudaFreeHost");
+  return PAC_SUCCESS;
+}
+int be_get_device() {
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess ? dev : 0;
+}
+void be_set_device(int device) { cudaSetDevice(device); }
+int be_sync_event_create(void** ev) {
+  cudaEvent_t e;
+  PAC_CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+  *ev = e;
+  return PAC_SUCCESS;
+}
+int be_event_wait(void* ev) {
+  PAC_CU(cudaEventSynchronize((cudaEvent_t)ev), "cudaEventSynchronize");
+  return PAC_SUCCESS;
+}
+
 int be_memcpy(void* dst, const void* src, size_t bytes, int kind, void* stream) {
   if (!bytes) return PAC_SUCCESS;
   cudaMemcpyKind k = kind == CPY_H2D   ? cudaMemcpyHostToDevice

@@ -40,6 +40,15 @@ int be_free(void* p) {
   free(p);
   return PAC_SUCCESS;
 }
+int be_host_alloc(void** p, size_t bytes) { return be_malloc(p, bytes); }
+int be_host_free(void* p) { return be_free(p); }
+int be_get_device() { return 0; }
+void be_set_device(int) {}
+int be_sync_event_create(void** ev) {
+  *ev = new double(0.0);
+  return PAC_SUCCESS;
+}
+int be_event_wait(void*) { return PAC_SUCCESS; }
 int be_memcpy(void* dst, const void* src, size_t bytes, int, void*) {
   if (bytes && dst != src) memmove(dst, src, bytes);
   return PAC_SUCCESS;

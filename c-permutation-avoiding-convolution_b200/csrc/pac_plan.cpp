@@ -39,6 +39,7 @@
 
 #include "pac.h"
 #include "pac_backend.h"
+#include "pac_host.h"
 #include "pac_special.h"
 #include "pac_vec_list.h"
 
@@ -1530,5 +1531,18 @@ PAC_API const char* pac_status_string(int status) {
 }
 
 PAC_API const char* pac_last_error(void) { return t_err; }
+
+// pac_host.h
+int pac_host_alloc(void** p, size_t bytes) { return be_host_alloc(p, bytes); }
+void pac_host_free(void* p) { be_host_free(p); }
+int pac_host_device(void) { return be_get_device(); }
+void pac_host_set_device(int device) { be_set_device(device); }
+int pac_host_event_create(void** ev) { return be_sync_event_create(ev); }
+void pac_host_event_destroy(void* ev) { be_event_destroy(ev); }
+int pac_host_event_record(void* ev, pac_stream_t stream) { return be_event_record(ev, stream); }
+int pac_host_event_wait(void* ev) { return be_event_wait(ev); }
+int pac_host_fetch_status(pac_plan_t plan, int* word, pac_stream_t stream) {
+  return be_memcpy(word, plan->status, sizeof(int), CPY_D2H, stream);
+}
 
 }  // extern "C"
