@@ -506,11 +506,16 @@ static EnvChoice env_choice() {
 
 // Switch a pass to the kernel over 8-byte elements (pac_vec.cuh) of its
 // geometry.  Plans with knobs and the environment's kernel choices keep the
-// kernels those select, the tensor-core form its own; a column tile has to
+// kernels those select; a column tile has to
 // lie within the stride, and the copies want 16-byte aligned arrays.
 static bool apply_vec(const Schedule& s, PassSpec& p, const EnvChoice& env) {
   PassDesc& d = p.d;
-  if (s.special != 0 || s.w_shift != 0 || s.rlog_cap < 4 || d.tc || d.plane) return false;
+  if (s.special != 0 || s.w_shift != 0 || s.rlog_cap < 4 || d.plane) return false;
+  // the tensor-core form's radix-16 stages have kernels of their own; a pass
+  // without one is FP32 in either form
+  if (d.tc)
+    for (int i = 0; i < d.nst; ++i)
+      if (d.rlog[i] == 4) return false;
   if (env.coltma || env.pipe || env.cluster || env.special) return false;
   const int cols = d.logS > 0 ? 1 : 0;
   VecGeo g;

@@ -180,3 +180,19 @@ def test_spectrum_replay(emu, dims, nf, base, tune, form):
 @pytest.mark.parametrize("dims,nf,base,tune", SPECTRA)
 def test_spectrum_gpu(lib, dims, nf, base, tune, form):
     check_spectrum(lib, dims, nf, base, tune, form)
+
+
+# tensor-core plans: passes without a radix-16 stage run here, the others on
+# the tensor cores, in one plan (64 x 256: the columns here, the rows there)
+TC = [((64, 512), 1, 2), ((8, 64, 32), 2, 2), ((8 ** 4,), 3, 8), ((64, 256), 1, 2), ((512, 16), 3, 2)]
+
+
+@pytest.mark.parametrize("dims,batch,base", TC)
+def test_tc_replay(emu, orc, dims, batch, base):
+    P.check_tc(emu, orc, dims, batch, base, ops=len(dims) < 3 and base == 2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims,batch,base", TC)
+def test_tc_gpu(lib, orc, dims, batch, base):
+    P.check_tc(lib, orc, dims, batch, base, ops=len(dims) < 3 and base == 2)
