@@ -21,6 +21,7 @@ int be_malloc(void** p, size_t bytes);
 int be_free(void* p);
 int be_host_alloc(void** p, size_t bytes);  // pinned host memory
 int be_host_free(void* p);
+int be_host_kind(const void* p);  // 0 ordinary, 1 pinned, 2 device or managed
 int be_get_device();
 void be_set_device(int device);
 int be_sync_event_create(void** ev);  // no timing, its waiter sleeps

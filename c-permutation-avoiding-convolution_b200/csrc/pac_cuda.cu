@@ -510,6 +510,14 @@ int be_host_free(void* p) {
   if (p) PAC_CU(cudaFreeHost(p), "cudaFreeHost");
   return PAC_SUCCESS;
 }
+int be_host_kind(const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return a.type == cudaMemoryTypeUnregistered ? 0 : a.type == cudaMemoryTypeHost ? 1 : 2;
+}
 int be_get_device() {
   int dev = 0;
   return cudaGetDevice(&dev) == cudaSuccess ? dev : 0;

@@ -98,6 +98,7 @@ typedef struct {
   int* rho;        /* device: N ints (permutation-only paths) */
   char* pin;       /* pinned: staging of a small entry's arrays, status word */
   int pooled;      /* a large entry: holds a reference on the staging pool */
+  int staged;      /* this call goes through pin */
   pac_stream_t s1, s2;
   unsigned long long last_use;
   pthread_mutex_t mu;
@@ -107,6 +108,8 @@ typedef struct {
 /* host copies.  The driver stages an ordinary host array through its own   */
 /* pinned buffer with one thread (32 MB in: 3.2 ms, out 1.8 to 2.9, where    */
 /* the bus takes 0.6) and synchronises on the way out.                      */
+/* Pinned arrays of large calls, and memory that the host does not own alone,  */
+/* are copied as they are.                                                    */
 /*   small entries (all arrays within SMALL_BYTES): one pinned block per     */
 /*   entry, one copy in and one out per call;                               */
 /*   large entries: a pool of pinned slots, filled and emptied by a few      */
@@ -151,6 +154,7 @@ typedef struct {
   int in;           /* 1 host -> device, 0 device -> host */
   pac_stream_t stream;
   int device;
+  size_t chunk;        /* bytes of one, at most a slot */
   size_t chunks, next; /* next: atomic */
   int status;
   char* pin;
@@ -165,7 +169,7 @@ static void* copy_worker(void* arg) {
   worker_t* w = (worker_t*)arg;
   copy_t* c = w->c;
   pac_host_set_device(c->device);
-  const size_t per = (c->nb + SLOT_BYTES - 1) / SLOT_BYTES; /* chunks of one array */
+  const size_t per = (c->nb + c->chunk - 1) / c->chunk; /* chunks of one array */
   void* ev[THREAD_SLOTS] = {NULL};
   char* out[THREAD_SLOTS] = {NULL}; /* where a slot's chunk has to go */
   size_t len[THREAD_SLOTS] = {0};
@@ -186,8 +190,8 @@ static void* copy_worker(void* arg) {
       if (!left) break;
       continue;
     }
-    const size_t a = q / per, off = (q % per) * SLOT_BYTES;
-    len[k] = c->nb - off < SLOT_BYTES ? c->nb - off : SLOT_BYTES;
+    const size_t a = q / per, off = (q % per) * c->chunk;
+    len[k] = c->nb - off < c->chunk ? c->nb - off : c->chunk;
     char* dev = (char*)c->dev + a * c->nb + off;
     char* host = (char*)c->host[a] + off;
     if (c->in) {
@@ -209,11 +213,11 @@ static void* copy_worker(void* arg) {
 }
 
 /* both arrays of a pair between host and device (dev: re|im back to back),
- * in stream order; out: on return the host has them, in: the host arrays may
- * be overwritten */
+ * in stream order; out: the host has them after finish() */
 static int copy_pair(double* dev, double* re, double* im, size_t nb, int in, pac_stream_t stream) {
   int st;
-  if (!g_pool.pin || pthread_mutex_trylock(&g_pool.busy) != 0) {
+  const int direct = pac_host_kind(re) != 0 && pac_host_kind(im) != 0;
+  if (direct || !g_pool.pin || pthread_mutex_trylock(&g_pool.busy) != 0) {
     if (in) {
       st = pac_memcpy_h2d(dev, re, nb, stream);
       if (st == PAC_SUCCESS) st = pac_memcpy_h2d((char*)dev + nb, im, nb, stream);
@@ -221,11 +225,13 @@ static int copy_pair(double* dev, double* re, double* im, size_t nb, int in, pac
       st = pac_memcpy_d2h(re, dev, nb, stream);
       if (st == PAC_SUCCESS) st = pac_memcpy_d2h(im, (char*)dev + nb, nb, stream);
     }
-    if (st == PAC_SUCCESS) st = pac_stream_synchronize(stream);
-    return st;
+    if (st == PAC_SUCCESS && !direct) st = pac_stream_synchronize(stream);
+    return st; /* (direct: the copies are queued, finish() waits) */
   }
-  copy_t c = {dev, {re, im}, nb, in, stream, pac_host_device(), 0, 0, PAC_SUCCESS, g_pool.pin};
-  c.chunks = 2 * ((nb + SLOT_BYTES - 1) / SLOT_BYTES);
+  copy_t c = {dev, {re, im}, nb, in, stream, pac_host_device(), 0, 0, 0, PAC_SUCCESS, g_pool.pin};
+  /* a quarter of an array, 256 KiB to a slot */
+  c.chunk = nb / 4 > SLOT_BYTES ? SLOT_BYTES : nb / 4 < SLOT_BYTES / 4 ? SLOT_BYTES / 4 : nb / 4;
+  c.chunks = 2 * ((nb + c.chunk - 1) / c.chunk);
   long cpus = sysconf(_SC_NPROCESSORS_ONLN);
   size_t n = c.chunks / 2 < COPY_THREADS ? c.chunks / 2 : COPY_THREADS;
   if (cpus > 0 && n > (size_t)cpus) n = (size_t)cpus;
@@ -384,9 +390,14 @@ static void release(entry_t* e) {
 /* arrays into the device pairs x (and h), and results back.  Small entries:
  * through their pinned block, the host arrays written once everything has
  * arrived (finish).  Large ones: straight into the host arrays. */
+static void choose_staging(entry_t* e, double* re, double* im, double* h_re, double* h_im) {
+  e->staged = e->pin && pac_host_kind(re) < 2 && pac_host_kind(im) < 2 &&
+              (!h_re || (pac_host_kind(h_re) < 2 && pac_host_kind(h_im) < 2));
+}
 static int arrays_in(entry_t* e, double* re, double* im, double* h_re, double* h_im) {
   const size_t nb = (size_t)e->N * sizeof(double);
-  if (!e->pin) {
+  choose_staging(e, re, im, h_re, h_im);
+  if (!e->staged) {
     int st = copy_pair(e->x, re, im, nb, 1, e->s1);
     if (st == PAC_SUCCESS && h_re) st = copy_pair(e->h, h_re, h_im, nb, 1, e->s1);
     return st;
@@ -402,7 +413,7 @@ static int arrays_in(entry_t* e, double* re, double* im, double* h_re, double* h
 /* a pair back: the first call for x, another for h */
 static int pair_out(entry_t* e, double* dev, double* re, double* im) {
   const size_t nb = (size_t)e->N * sizeof(double);
-  if (!e->pin) return copy_pair(dev, re, im, nb, 0, e->s1);
+  if (!e->staged) return copy_pair(dev, re, im, nb, 0, e->s1);
   return pac_memcpy_d2h(e->pin + (dev == e->x ? 0 : 2 * nb), dev, 2 * nb, e->s1);
 }
 /* waits; a device wait that gave up is reported; then a small entry's host
@@ -410,7 +421,7 @@ static int pair_out(entry_t* e, double* dev, double* re, double* im) {
 static int finish(entry_t* e, double* re, double* im, double* h_re, double* h_im) {
   const size_t nb = (size_t)e->N * sizeof(double);
   int st = PAC_SUCCESS;
-  if (!e->pin) {
+  if (!e->staged) {
     st = pac_stream_synchronize(e->s1);
     if (st == PAC_SUCCESS && e->plan) st = pac_plan_check_status(e->plan, e->s1);
     return st;
@@ -516,7 +527,8 @@ static void run_pac_conv(const char* fn, int rank, const int* dims, int r, doubl
    * copy is what the convolution reads.  A large entry's filter arrives and
    * is transformed while its signal is copied, and leaves while the
    * convolution runs. */
-  if (e->pin) {
+  choose_staging(e, re, im, h_re, h_im);
+  if (e->staged) {
     TRY(arrays_in(e, re, im, h_re, h_im));
     TRY(pac_transform(e->plan, PAC_OP_AT, hr, hi, hr, hi, e->s1));
   } else {
@@ -525,11 +537,11 @@ static void run_pac_conv(const char* fn, int rank, const int* dims, int r, doubl
     TRY(copy_pair(e->x, re, im, nb, 1, e->s2));
     TRY(pac_stream_wait_stream(e->s2, e->s1));
   }
-  pac_stream_t s = e->pin ? e->s1 : e->s2;
+  pac_stream_t s = e->staged ? e->s1 : e->s2;
   TRY(pac_spectrum_to_plan_order(e->plan, hr, hi, 1, e->hhat, e->hhat + N, 1.0, s));
   TRY(pac_convolve(e->plan, xr, xi, e->hhat, e->hhat + N, 0, xr, xi, 1.0 / (double)N, s));
   TRY(pair_out(e, e->h, h_re, h_im));
-  if (!e->pin) TRY(pac_stream_wait_stream(e->s1, e->s2));
+  if (!e->staged) TRY(pac_stream_wait_stream(e->s1, e->s2));
   TRY(pair_out(e, e->x, re, im));
   TRY(finish(e, re, im, h_re, h_im));
 done:

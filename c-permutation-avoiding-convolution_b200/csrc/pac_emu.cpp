@@ -42,6 +42,7 @@ int be_free(void* p) {
 }
 int be_host_alloc(void** p, size_t bytes) { return be_malloc(p, bytes); }
 int be_host_free(void* p) { return be_free(p); }
+int be_host_kind(const void*) { return 0; }
 int be_get_device() { return 0; }
 void be_set_device(int) {}
 int be_sync_event_create(void** ev) {

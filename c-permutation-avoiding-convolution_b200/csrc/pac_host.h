@@ -16,6 +16,8 @@ int pac_host_alloc(void** p, size_t bytes); /* pinned, for every device */
 void pac_host_free(void* p);
 int pac_host_device(void);            /* the calling thread's device ... */
 void pac_host_set_device(int device); /* ... for a thread it started */
+/* 0 ordinary host memory, 1 pinned, 2 not host memory alone (device, managed) */
+int pac_host_kind(const void* p);
 int pac_host_event_create(void** ev);
 void pac_host_event_destroy(void* ev);
 int pac_host_event_record(void* ev, pac_stream_t stream);

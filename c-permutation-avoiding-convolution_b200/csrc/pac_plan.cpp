@@ -1540,6 +1540,7 @@ PAC_API const char* pac_last_error(void) { return t_err; }
 // pac_host.h
 int pac_host_alloc(void** p, size_t bytes) { return be_host_alloc(p, bytes); }
 void pac_host_free(void* p) { be_host_free(p); }
+int pac_host_kind(const void* p) { return be_host_kind(p); }
 int pac_host_device(void) { return be_get_device(); }
 void pac_host_set_device(int device) { be_set_device(device); }
 int pac_host_event_create(void** ev) { return be_sync_event_create(ev); }
