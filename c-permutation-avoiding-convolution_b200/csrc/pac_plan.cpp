@@ -1328,12 +1328,14 @@ PAC_API int pac_filter_spectrum(pac_plan_t plan, const double* h_re, const doubl
   // F32 form: FP64 transform, reordered and rounded once
   std::lock_guard<std::mutex> g(plan->ws_mu);
   const bool direct = spectrum_direct(plan, *plan->s64);
-  // (one pass reads h while it writes hhat: not where they share memory)
+  const bool one_pass = plan->s64->vax.size() == 1;
+  // (one pass reads h while it writes hhat: not where they share memory.  Of
+  // several passes the last reads the temporary)
   const size_t hb = (size_t)nfilters * plan->N;
   auto apart = [&](const double* a, void* b) {
     return (char*)b >= (char*)(a + hb) || (char*)a >= (char*)b + hb * sizeof(float);
   };
-  if (direct && plan->s64->vax.size() == 1 && apart(h_re, hhat_re) && apart(h_re, hhat_im) &&
+  if (direct && one_pass && apart(h_re, hhat_re) && apart(h_re, hhat_im) &&
       apart(h_im, hhat_re) && apart(h_im, hhat_im)) {
     int done = 0;
     PAC_TRY(run_spectrum(plan, *plan->s64, nfilters, h_re, h_im, hhat_re, hhat_im, nullptr,
@@ -1350,7 +1352,7 @@ PAC_API int pac_filter_spectrum(pac_plan_t plan, const double* h_re, const doubl
   }
   double* tre = (double*)plan->tmp64;
   double* tim = tre + (size_t)nfilters * plan->N;
-  if (direct) {
+  if (direct && !one_pass) {
     int done = 0;
     PAC_TRY(run_spectrum(plan, *plan->s64, nfilters, h_re, h_im, hhat_re, hhat_im, tre, tim, scale,
                          stream, &done));
