@@ -405,6 +405,33 @@ static int replay_plane(const PassDesc& d, long long grid) {
   return PAC_SUCCESS;
 }
 
+// A pass over 8-byte elements may start before the launch ahead of it has
+// ended (pac_vec.cu), so its arrays may still be written while it runs and
+// must not be read through the read-only path: such loads are counted.
+struct DataRange {
+  const char *lo = nullptr, *hi = nullptr;
+};
+static thread_local DataRange g_data[6];
+static std::atomic<long long> g_read_only_data{0};
+void emu_read_only_load(const void* p) {
+  for (const DataRange& r : g_data)
+    if ((const char*)p >= r.lo && (const char*)p < r.hi) g_read_only_data++;
+}
+static void set_data_ranges(const PassDesc& d, int elem_bytes) {
+  long long n = d.nlines << d.logL;  // elements
+  if (d.poff) {
+    n = 0;
+    const long long per = 1LL << (d.logLP + d.logL);
+    for (long long p = 0; p < d.nlines >> d.logLP; ++p) n = std::max(n, d.poff[p] + per);
+  }
+  const long long nh = d.mode != MODE_CONV ? 0 : d.h_mask == -1 ? n : d.h_mask + 1;
+  const void* at[6] = {d.in_re, d.in_im, d.out_re, d.out_im, d.h_re, d.h_im};
+  for (int k = 0; k < 6; ++k) {
+    const long long bytes = (k < 4 ? n : nh) * (k == 2 || k == 3 ? d.porder ? d.porder : elem_bytes : elem_bytes);
+    g_data[k] = {(const char*)at[k], (const char*)at[k] + bytes};
+  }
+}
+
 // the passes over 8-byte elements (pac_emu_vec.cpp, sliced as pac_vec.cu)
 #define PAC_VEC_DECLARE(k) int replay_vec_##k(const PassDesc& d, int elem_bytes, int b2);
 PAC_VEC_DECLARE(0) PAC_VEC_DECLARE(1) PAC_VEC_DECLARE(2) PAC_VEC_DECLARE(3) PAC_VEC_DECLARE(4)
@@ -414,10 +441,12 @@ static int replay_vec(const PassDesc& d, int elem_bytes, int b2) {
       replay_vec_0, replay_vec_1, replay_vec_2, replay_vec_3, replay_vec_4,
       replay_vec_5, replay_vec_6, replay_vec_7, replay_vec_8, replay_vec_9};
   if (d.W * d.L > 0 && copy_wait_gives_up(d)) return PAC_SUCCESS;
-  for (auto f : fn) {
-    const int st = f(d, elem_bytes, b2);
-    if (st >= 0) return st;
-  }
+  set_data_ranges(d, elem_bytes);
+  int st = -1;
+  for (auto f : fn)
+    if (st < 0) st = f(d, elem_bytes, b2);
+  for (DataRange& r : g_data) r = DataRange();
+  if (st >= 0) return st;
   return set_error(PAC_ERROR_INTERNAL, "no replay for a pass over 8-byte elements");
 }
 
@@ -732,3 +761,9 @@ int be_graph_launch(void*, void*) {
 int be_graph_destroy(void*) { return PAC_SUCCESS; }
 
 }  // namespace pac
+
+// read by the tests: loads of a dependent launch's arrays through the
+// read-only path since the library was loaded
+extern "C" PAC_API long long pac_emu_read_only_data_loads(void) {
+  return pac::g_read_only_data.load();
+}

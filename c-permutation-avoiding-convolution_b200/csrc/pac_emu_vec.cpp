@@ -119,7 +119,7 @@ int cols_as(const PassDesc& d) {
 template <int B2, int MODE, int SIGN, int LOGL, int TW4, int OFFS>
 int small_as(const PassDesc& d) {
   for (long long u = 0; u < d.nlines / VT<V>::LPU; ++u)
-    VecSmall<V, B2, MODE, SIGN, LOGL, OFFS>::template run<TW4>(d, u);
+    VecSmall<V, B2, MODE, SIGN, LOGL, OFFS>::template run<TW4>(d, u, [] {});
   return PAC_SUCCESS;
 }
 

@@ -295,6 +295,15 @@ PAC_HD int sidx(int e) {
   return e + (e >> Pad<T>::SH);
 }
 
+// Loads through the read-only path: memory that nothing writes during the
+// kernel.  (The host replay checks them against a dependent launch's arrays.)
+#if defined(PAC_EMULATE)
+void emu_read_only_load(const void* p);  // pac_emu.cpp
+#define PAC_READ_ONLY(p) ::pac::emu_read_only_load(p)
+#else
+#define PAC_READ_ONLY(p) (void)0
+#endif
+
 template <typename T>
 PAC_HD Cx<T> ld_tw(const Cx<T>* p) {
 #if defined(__CUDA_ARCH__)
@@ -306,6 +315,7 @@ PAC_HD Cx<T> ld_tw(const Cx<T>* p) {
     return Cx<T>{v.x, v.y};
   }
 #else
+  PAC_READ_ONLY(p);
   return *p;
 #endif
 }
@@ -315,6 +325,7 @@ PAC_HD T ld_g(const T* p) {
 #if defined(__CUDA_ARCH__)
   return __ldg(p);
 #else
+  PAC_READ_ONLY(p);
   return *p;
 #endif
 }

@@ -108,24 +108,24 @@ PAC_HD V vnfma(V a, V b, V c) {
   return vfma(vneg(a), b, c);
 }
 
-// a read-only load that stays where it is written (ahead of a barrier)
+// Loads of signals, intermediates and filter spectra.  These passes may start
+// before the launch ahead of them has ended (pac_vec.cu), so what they read may
+// still be written while they run: ordinary loads, after pdl_wait.  (The
+// read-only path, __ldg, is for memory that nothing writes during the kernel:
+// the compiler may move such a load ahead of the wait, and its cache need not
+// see the writes.  It is left to the twiddle tables.)
+template <class V>
+PAC_HD V ld_data(const V* p) {
+  return *p;
+}
+// the same, staying where it is written (ahead of a barrier)
 template <class T>
 PAC_HD T ld_now(const T* p) {
 #if defined(__CUDA_ARCH__)
   T v;
-  if constexpr (sizeof(T) == 8) asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
-  else asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  if constexpr (sizeof(T) == 8) asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  else asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
   return v;
-#else
-  return *p;
-#endif
-}
-PAC_HD double vload(const double* p) { return ld_g(p); }
-PAC_HD F2 vload(const F2* p) {
-#if defined(__CUDA_ARCH__)
-  F2 r;
-  r.u = __ldg(reinterpret_cast<const unsigned long long*>(p));
-  return r;
 #else
   return *p;
 #endif
@@ -647,7 +647,7 @@ struct VecPass {
         constexpr int m = mm.value;
         constexpr int sl = dif_step(0) ? m : drev_c(m, LR, B2);
         const long long gi = base + ((long long)(e0 + (sl << logell)) << rowsh) + w;
-        x[kk.value * R + m] = {vload(ire + gi), vload(iim + gi)};
+        x[kk.value * R + m] = {ld_data(ire + gi), ld_data(iim + gi)};
       });
     });
   }
@@ -1016,8 +1016,9 @@ struct VecSmall {
   static constexpr int L = 1 << LOGL, LPU = VT<V>::LPU;
   static_assert(LOGL >= 1 && LOGL <= 4 && LOGL % B2 == 0 && (B2 != 3 || LOGL == 3), "one stage");
   // unit u of nlines / LPU
-  template <int TW4>
-  static PAC_HD void run(const PassDesc& d, long long u) {
+  // loaded() runs once the unit is in registers
+  template <int TW4, class F>
+  static PAC_HD void run(const PassDesc& d, long long u, F&& loaded) {
     const int su = d.logS - ilog2(LPU);
     const V* ire = (const V*)d.in_re;
     const V* iim = (const V*)d.in_im;
@@ -1036,8 +1037,9 @@ struct VecSmall {
     static_for<L>([&](auto mm) {
       constexpr int m = mm.value;
       const long long gi = in0 + ((long long)(MODE == MODE_DIF ? m : drev_c(m, LOGL, B2)) << su);
-      x[m] = {vload(ire + gi), vload(iim + gi)};
+      x[m] = {ld_data(ire + gi), ld_data(iim + gi)};
     });
+    loaded();
     if constexpr (TW4 && MODE == MODE_DIT) vtw4_apply<TW4, L, SIGN, B2, true>(d, u * LPU, 0, LOGL, x);
     vdft<L, SIGN>(x);
     if constexpr (TW4 && MODE == MODE_DIF) vtw4_apply<TW4, L, SIGN, B2, true>(d, u * LPU, 0, LOGL, x);

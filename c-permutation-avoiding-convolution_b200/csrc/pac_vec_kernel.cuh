@@ -181,8 +181,8 @@ template <class V, int B2, int MODE, int SIGN, int LOGL, int TW4, int OFFS>
 __global__ void __launch_bounds__(256) pac_vec_small_kernel(const __grid_constant__ PassDesc d) {
   const long long u = (long long)blockIdx.x * 256 + threadIdx.x;
   pdl_wait();
-  pdl_trigger();
-  if (u < d.nlines / VT<V>::LPU) VecSmall<V, B2, MODE, SIGN, LOGL, OFFS>::template run<TW4>(d, u);
+  if (u < d.nlines / VT<V>::LPU)
+    VecSmall<V, B2, MODE, SIGN, LOGL, OFFS>::template run<TW4>(d, u, [] { pdl_trigger(); });
 }
 
 }  // namespace pac
