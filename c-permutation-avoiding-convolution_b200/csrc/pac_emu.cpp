@@ -63,7 +63,13 @@ int be_stream_create(void** s) {
   return PAC_SUCCESS;
 }
 int be_stream_destroy(void*) { return PAC_SUCCESS; }
-int be_stream_sync(void*) { return PAC_SUCCESS; }
+// tables have been filled and nothing has waited for them yet
+static std::atomic<int> g_tables_pending{0};
+static std::atomic<long long> g_early_tables{0};
+int be_stream_sync(void*) {
+  g_tables_pending = 0;
+  return PAC_SUCCESS;
+}
 int be_stream_wait(void*, void*) { return PAC_SUCCESS; }
 int be_l2_persist(void*, const void*, size_t) { return PAC_SUCCESS; }
 long long be_l2_bytes() { return 0; }
@@ -453,6 +459,9 @@ static int replay_vec(const PassDesc& d, int elem_bytes, int b2) {
 int be_launch_pass(const PassDesc& d, int elem_bytes, int b2, long long grid, int threads,
                    size_t, void*) {
   if (d.vec == VEC_PREPARE) return PAC_SUCCESS;
+  // a launch that is not dependent waits for all that is queued ahead of it
+  if (d.vec && d.dependent) g_early_tables += g_tables_pending.load();
+  else g_tables_pending = 0;
   if (d.vec) {
     g_launches++;
     return replay_vec(d, elem_bytes, b2);
@@ -558,6 +567,7 @@ int be_fill_tc_const(void* dst, void*) {
 }
 
 int be_fill_stage_tw(void* dst, int elem_bytes, int logK, int logR, void*) {
+  g_tables_pending = 1;
   long long R1 = (1LL << logR) - 1, K = 1LL << logK;
   long long n = (K >> logR) * R1;
   for (long long idx = 0; idx < n; ++idx) {
@@ -574,6 +584,7 @@ int be_fill_stage_tw(void* dst, int elem_bytes, int logK, int logR, void*) {
 }
 
 int be_fill_pow_tw(void* dst, int elem_bytes, long long count, long long stride, int logN, void*) {
+  g_tables_pending = 1;
   long long N = 1LL << logN;
   for (long long k = 0; k < count; ++k) {
     double c, sn;
@@ -586,6 +597,7 @@ int be_fill_pow_tw(void* dst, int elem_bytes, long long count, long long stride,
 }
 
 int be_fill_tw4(void* dst, int elem_bytes, int logL, int logN, void*) {
+  g_tables_pending = 1;
   const long long N = 1LL << logN, M = N >> logL;
   for (long long q = 0; q < N; ++q) {
     double c, sn;
@@ -766,4 +778,22 @@ int be_graph_destroy(void*) { return PAC_SUCCESS; }
 // read-only path since the library was loaded
 extern "C" PAC_API long long pac_emu_read_only_data_loads(void) {
   return pac::g_read_only_data.load();
+}
+
+// read by the tests: dependent passes launched behind the filling of tables
+// that nothing had waited for
+extern "C" PAC_API long long pac_emu_early_tables(void) { return pac::g_early_tables.load(); }
+
+// pac_convolve_1d_noalloc over caller-supplied scratch
+namespace pac {
+int conv_in_scratch(void* scratch, size_t scratch_bytes, int logn, int batch, const double* x_re,
+                    const double* x_im, const double* h_re, const double* h_im, double* y_re,
+                    double* y_im, void* stream);
+}
+extern "C" PAC_API int pac_emu_conv_in_scratch(void* scratch, size_t bytes, int logn, int batch,
+                                               const double* x_re, const double* x_im,
+                                               const double* h_re, const double* h_im,
+                                               double* y_re, double* y_im) {
+  return pac::conv_in_scratch(scratch, bytes, logn, batch, x_re, x_im, h_re, h_im, y_re, y_im,
+                              nullptr);
 }

@@ -117,9 +117,11 @@ struct PassDesc {
   // 2^porder_logR positions transposed) in elements of porder bytes; 0: no
   int porder;
   int porder_logR;
-  // 1: the tables were complete when the plan was handed out, so a kernel may
-  // read them ahead of the work queued before it
-  int tw_fixed;
+  // vec passes: the launch may start while the work queued ahead of it still
+  // runs, and then reads its twiddle tables at once.  Only where those were
+  // complete before that work began: the tables of a plan that was handed out,
+  // or those that an earlier pass of the call has already used
+  int dependent;
   // 1: plane pass of a 3D convolution (pac_plane.cuh): axes 1 and 2 of
   // every plane, whose stages are rlog[0 .. plane_n1s-1] (axis 1) then
   // rlog[plane_n1s .. nst-1] (axis 2), on a cluster of 2^logC CTAs

@@ -704,7 +704,8 @@ static int exec_passes(pac_plan_s* pl, const Schedule& s, std::vector<PassSpec>&
   for (auto& p : passes) {
     p.d.status = pl->status;
     p.d.wait_limit = pl->wait_limit;
-    p.d.tw_fixed = s.tables_fixed;
+    // (the first pass over tables filled on this stream waits for them)
+    p.d.dependent = s.tables_fixed || &p != &passes[0];
     apply_special(s, p, env);
   }
   if (!pl->timing) {
@@ -1068,7 +1069,7 @@ int plan_batch_passes(pac_plan_s* pl, long long copies, const long long* poff, c
     p.d.poff = poff;
     p.d.logLP = logN - p.d.logL;
     p.d.status = pl->status;
-    p.d.tw_fixed = s.tables_fixed;
+    p.d.dependent = s.tables_fixed;
     descs.push_back(p.d);
     tiles.push_back(p.grid);
   }

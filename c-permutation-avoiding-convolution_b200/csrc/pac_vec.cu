@@ -72,9 +72,10 @@ int resident(Resident& r, K kern, int nt, size_t smem, long long* out) {
 // over the SMs: CTAs that arrive while the kernel before still runs would
 // otherwise pile up on the SMs that it leaves first, so each reserves its
 // share of an SM's shared memory.
+// (A pass that may not start early, PassDesc.dependent, is launched plainly.)
 template <class K, class... A>
 int pdl_launch(K kern, long long tiles, long long slots, int nt, size_t smem, cudaStream_t st,
-               const A&... args) {
+               const PassDesc& d, const A&... args) {
   const long long fit = slots < 0 ? -slots : slots;
   long long grid = tiles;
   if (slots > 0 && tiles > slots) grid = slots;
@@ -93,8 +94,8 @@ int pdl_launch(K kern, long long tiles, long long slots, int nt, size_t smem, cu
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
-  PAC_CU(cudaLaunchKernelEx(&cfg, kern, args...), "pass over 8-byte elements");
+  cfg.numAttrs = d.dependent ? 1 : 0;
+  PAC_CU(cudaLaunchKernelEx(&cfg, kern, d, args...), "pass over 8-byte elements");
   count_launch();
   return PAC_SUCCESS;
 }

@@ -67,9 +67,8 @@ __device__ __forceinline__ void vec_tiles(const PassDesc& d, CV<V>* B, uint64_t*
   }
   using Real = typename VP::Real;
   Cx<Real>* tws = reinterpret_cast<Cx<Real>*>(B + VP::TILE);
-  if (!d.tw_fixed) pdl_wait();
   VP::tw_fill(d, threadIdx.x, tws);  // read after the first tile's barrier
-  if (d.tw_fixed) pdl_wait();
+  pdl_wait();
   __syncthreads();
   long long tile = blockIdx.x;
   if (threadIdx.x == 0 && tile < ntiles) issue(tile);

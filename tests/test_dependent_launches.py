@@ -6,6 +6,8 @@ loads that fall into a pass's own arrays.  On the GPU, calls queued without a
 wait -- one-stage columns, bases 4 and 8, spectra of changing filters read at
 once by the pass that follows -- give bit for bit what the same calls give
 when each is waited for."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -82,3 +84,40 @@ def test_queued_calls(lib, dims, batch, base, form):
     for u, v in zip(a, b):
         assert np.isfinite(u).all()
         assert np.array_equal(u, v)
+
+
+# the no-allocation entry point fills its tables on the caller's stream, so
+# the first pass over them may not start early; the largest and the smallest
+# sizes, and the one whose split depends on the batch
+NOALLOC = [(6, 5), (12, 3), (13, 3), (13, 70), (14, 2), (15, 1), (16, 2)]
+SCRATCH = 1280 * 1024  # its static array
+
+
+@pytest.mark.parametrize("logn,batch", NOALLOC)
+def test_tables_are_waited_for(emu, logn, batch):
+    n = 1 << logn
+    g = rng(logn)
+    x = g.standard_normal((batch, n)) + 1j * g.standard_normal((batch, n))
+    h = g.standard_normal(n) + 1j * g.standard_normal(n)
+    d = P.Dev(emu)
+    emu.pac_emu_conv_in_scratch.argtypes = [C.c_void_p, C.c_size_t, C.c_int, C.c_int] + [C.c_void_p] * 6
+    before = emu.pac_emu_early_tables()
+    try:
+        a = [d.put(np.ascontiguousarray(v)) for v in (x.real, x.imag, h.real, h.imag)]
+        y = [d.zeros((batch, n), np.float64) for _ in range(2)]
+        scratch = d.put(np.full(SCRATCH, 255, np.uint8))  # NaN
+        for _ in range(2):
+            pac.check(emu, emu.pac_emu_conv_in_scratch(scratch, SCRATCH, logn, batch, *a, *y), "conv")
+        y = [d.get(p, (batch, n), np.float64) for p in y]
+    finally:
+        d.free()
+    assert P.crel(y[0] + 1j * y[1], np.fft.ifft(np.fft.fft(x) * np.fft.fft(h))) < P.TOL
+    assert emu.pac_emu_early_tables() == before
+
+
+@pytest.mark.parametrize("form", [F64, F32])
+def test_plan_tables_are_waited_for(emu, form):
+    before = emu.pac_emu_early_tables()
+    convolutions(emu, (1 << 14,), 2, 2, form, False)
+    P.check_multi(emu, [(256,), (1 << 14,), (8, 256)], form)
+    assert emu.pac_emu_early_tables() == before
