@@ -99,6 +99,9 @@ def _declare(L):
     L.pac_multi_offsets.argtypes = [_vp, C.POINTER(ll)]
     L.pac_multi_filter_spectra.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp]
     L.pac_multi_convolve.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]
+    L.pac_multi_set_wait_limit.argtypes = [_vp, ll]
+    L.pac_multi_check_status.argtypes = [_vp, _vp]
+    L.pac_noalloc_check_status.argtypes = [_vp]
     L.pac_multi_get_info.argtypes = [_vp, C.POINTER(MultiInfo)]
     L.pac_multi_set_level_timing.argtypes = [_vp, i]
     L.pac_status_string.restype = C.c_char_p

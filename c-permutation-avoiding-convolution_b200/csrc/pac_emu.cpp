@@ -21,6 +21,7 @@
 #include "pac.h"
 #include "pac_backend.h"
 #include "pac_special.h"
+#include "pac_vec_list.h"
 
 namespace pac {
 
@@ -446,7 +447,13 @@ static int replay_vec(const PassDesc& d, int elem_bytes, int b2) {
   static int (*const fn[])(const PassDesc&, int, int) = {
       replay_vec_0, replay_vec_1, replay_vec_2, replay_vec_3, replay_vec_4,
       replay_vec_5, replay_vec_6, replay_vec_7, replay_vec_8, replay_vec_9};
-  if (d.W * d.L > 0 && copy_wait_gives_up(d)) return PAC_SUCCESS;
+  // (columns read straight from global memory have no copies to wait for)
+  VecGeo g;
+  const int cols = d.logS > 0 ? 1 : 0;
+  const bool direct = cols && (d.poff || vec_direct(d.mode, d.logL, d.tw4));
+  if (vec_geometry(b2, d.mode, d.sign, d.logL, cols, &g) && !g.small && !direct &&
+      copy_wait_gives_up(d))
+    return PAC_SUCCESS;
   set_data_ranges(d, elem_bytes);
   int st = -1;
   for (auto f : fn)
@@ -788,12 +795,21 @@ extern "C" PAC_API long long pac_emu_early_tables(void) { return pac::g_early_ta
 namespace pac {
 int conv_in_scratch(void* scratch, size_t scratch_bytes, int logn, int batch, const double* x_re,
                     const double* x_im, const double* h_re, const double* h_im, double* y_re,
-                    double* y_im, void* stream);
+                    double* y_im, int* status, long long wait_limit, void* stream);
+static int g_noalloc_status = PAC_SUCCESS;
+static long long g_noalloc_limit = 0;
+int noalloc_status_word(int** word) {
+  *word = &g_noalloc_status;
+  return PAC_SUCCESS;
+}
+}  // namespace pac
+extern "C" PAC_API void pac_emu_noalloc_wait_limit(long long cycles) {
+  pac::g_noalloc_limit = cycles;
 }
 extern "C" PAC_API int pac_emu_conv_in_scratch(void* scratch, size_t bytes, int logn, int batch,
                                                const double* x_re, const double* x_im,
                                                const double* h_re, const double* h_im,
                                                double* y_re, double* y_im) {
   return pac::conv_in_scratch(scratch, bytes, logn, batch, x_re, x_im, h_re, h_im, y_re, y_im,
-                              nullptr);
+                              &pac::g_noalloc_status, pac::g_noalloc_limit, nullptr);
 }

@@ -47,6 +47,8 @@ int plan_bytes(pac_plan_s* pl);
 int plan_batch_passes(pac_plan_s* pl, long long copies, const long long* poff, const void* x_re,
                       const void* x_im, const void* h_re, const void* h_im, void* y_re,
                       void* y_im, std::vector<PassDesc>& descs, std::vector<long long>& tiles);
+void plan_set_status_word(pac_plan_s* pl, int* word);
+int check_status_word(int* status, const char* what, void* stream);
 int plan_create_for_batch(pac_plan_t* plan, int rank, const int* dims, const int* bases, int form);
 }  // namespace pac
 
@@ -105,7 +107,11 @@ struct pac_multi_s {
   void* side = nullptr;  // second stream for the small-tile groups
   std::vector<Chain> chains;        // largest first
   void* lanes[kStreams] = {};       // streams 1 .. of the chains (0 is the caller's)
-  void* offs = nullptr;             // device: element offsets of the chains' problems
+  // device: the status word of the shapes' plans (256 bytes), then the element
+  // offsets of the chains' problems
+  void* offs = nullptr;
+  enum { kStatusBytes = 256 };
+  const long long* offsets() const { return (const long long*)((char*)offs + kStatusBytes); }
   std::vector<size_t> offs_at;      // per shape: its first offset
   std::vector<long long> copies;    // per shape: its problems
   int calls = 0;                    // with the current buffer set
@@ -153,7 +159,7 @@ static int build_levels(pac_multi_s* m, const void* x_re, const void* x_im, cons
   for (size_t k = 0; k < m->plans.size(); ++k) {
     Chain c;
     if (chained[k])
-      PAC_TRY(plan_batch_passes(m->plans[k], m->copies[k], (const long long*)m->offs + m->offs_at[k],
+      PAC_TRY(plan_batch_passes(m->plans[k], m->copies[k], m->offsets() + m->offs_at[k],
                                 x_re, x_im, h_re, h_im, y_re, y_im, c.d, c.tiles));
     chained[k] = !c.d.empty();
     if (c.d.empty()) continue;
@@ -410,9 +416,13 @@ static int create_multi(pac_multi_t* multi, int nprob, const int* ranks, const i
   std::vector<long long> host((size_t)nprob);
   std::vector<size_t> at = m->offs_at;
   for (int p = 0; p < nprob; ++p) host[at[m->shape_of[p]]++] = m->off[p];
-  PAC_TRY(be_malloc(&m->offs, sizeof(long long) * host.size()));
-  PAC_TRY(be_memcpy(m->offs, host.data(), sizeof(long long) * host.size(), CPY_H2D, nullptr));
+  PAC_TRY(be_malloc(&m->offs, pac_multi_s::kStatusBytes + sizeof(long long) * host.size()));
+  PAC_TRY(be_memset(m->offs, 0, pac_multi_s::kStatusBytes, nullptr));
+  PAC_TRY(be_memcpy((void*)m->offsets(), host.data(), sizeof(long long) * host.size(), CPY_H2D,
+                    nullptr));
   PAC_TRY(be_stream_sync(nullptr));
+  // one status word for every shape: its waits and those of its spectra
+  for (pac_plan_t p : m->plans) plan_set_status_word(p, (int*)m->offs);
   *multi = m.release();
   return PAC_SUCCESS;
 }
@@ -526,6 +536,19 @@ PAC_API int pac_multi_get_info(pac_multi_t m, pac_multi_info_t* info) {
   for (size_t k = 0; k < m->depth && k < kInfoLevels; ++k)
     info->level_ms[k] = m->timed_calls ? m->level_ms[k] / (double)m->timed_calls : 0.0;
   return PAC_SUCCESS;
+}
+
+PAC_API int pac_multi_set_wait_limit(pac_multi_t m, long long cycles) {
+  if (!m) return set_error(PAC_ERROR_INVALID_VALUE, "pac_multi_set_wait_limit: NULL multi-plan");
+  std::lock_guard<std::mutex> g(m->mu);
+  for (pac_plan_t p : m->plans) PAC_TRY(pac_plan_set_wait_limit(p, cycles));
+  m->built = false;  // the limit is in the recorded launches
+  return PAC_SUCCESS;
+}
+
+PAC_API int pac_multi_check_status(pac_multi_t m, pac_stream_t stream) {
+  if (!m) return set_error(PAC_ERROR_INVALID_VALUE, "pac_multi_check_status: NULL multi-plan");
+  return check_status_word((int*)m->offs, "this multi-plan", stream);
 }
 
 PAC_API int pac_multi_set_level_timing(pac_multi_t m, int enable) {

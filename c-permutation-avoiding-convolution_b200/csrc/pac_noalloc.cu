@@ -11,7 +11,7 @@
 //
 // The array is shared by all calls on a device and keeps the last call's
 // contents.  Every call rewrites all of it that it reads (twiddle tables and
-// filter spectrum) before reading it, so nothing needs clearing, but two
+// filter spectrum; the status word is only ever set) before reading it, so nothing needs clearing, but two
 // calls whose device work overlaps in time (different streams, or different
 // host threads) race on it.
 #include <cuda_runtime.h>
@@ -25,11 +25,15 @@ int set_error(int status, const char* fmt, ...);
 int be_init();
 int conv_in_scratch(void* scratch, size_t scratch_bytes, int logn, int batch, const double* x_re,
                     const double* x_im, const double* h_re, const double* h_im, double* y_re,
-                    double* y_im, void* stream);
+                    double* y_im, int* status, long long wait_limit, void* stream);
+int noalloc_status_word(int** word);
 }  // namespace pac
 
-// filter spectrum (2 x 2^16 doubles = 1 MiB) plus twiddle tables (< 64 KiB)
+// filter spectrum (2 x 2^16 doubles = 1 MiB) plus twiddle tables (at most 128
+// KiB, for rows of 8192 points); the last 256 bytes are the status word of the
+// bounded waits (pac_noalloc_check_status), which starts as PAC_SUCCESS
 #define PAC_NOALLOC_SCRATCH_BYTES (1280 * 1024)
+#define PAC_NOALLOC_STATUS_BYTES 256
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[PAC_NOALLOC_SCRATCH_BYTES];
 
@@ -58,6 +62,14 @@ static int scratch_on_current_device(void** out) {
   return PAC_SUCCESS;
 }
 
+int pac::noalloc_status_word(int** word) {
+  void* scratch = nullptr;
+  const int st = scratch_on_current_device(&scratch);
+  if (st == PAC_SUCCESS)
+    *word = (int*)((char*)scratch + PAC_NOALLOC_SCRATCH_BYTES - PAC_NOALLOC_STATUS_BYTES);
+  return st;
+}
+
 extern "C" PAC_API int pac_convolve_1d_noalloc(const double* x_re, const double* x_im,
                                                const double* h_re, const double* h_im,
                                                double* y_re, double* y_im, int n, int batch,
@@ -80,6 +92,9 @@ extern "C" PAC_API int pac_convolve_1d_noalloc(const double* x_re, const double*
   void* scratch = nullptr;
   st = scratch_on_current_device(&scratch);
   if (st != PAC_SUCCESS) return st;
-  return pac::conv_in_scratch(scratch, PAC_NOALLOC_SCRATCH_BYTES, logn, batch, x_re, x_im, h_re,
-                              h_im, y_re, y_im, stream);
+  int* status = nullptr;
+  st = pac::noalloc_status_word(&status);
+  if (st != PAC_SUCCESS) return st;
+  return pac::conv_in_scratch(scratch, PAC_NOALLOC_SCRATCH_BYTES - PAC_NOALLOC_STATUS_BYTES, logn,
+                              batch, x_re, x_im, h_re, h_im, y_re, y_im, status, 0, stream);
 }

@@ -1069,6 +1069,7 @@ int plan_batch_passes(pac_plan_s* pl, long long copies, const long long* poff, c
     p.d.poff = poff;
     p.d.logLP = logN - p.d.logL;
     p.d.status = pl->status;
+    p.d.wait_limit = pl->wait_limit;
     p.d.dependent = s.tables_fixed;
     descs.push_back(p.d);
     tiles.push_back(p.grid);
@@ -1076,6 +1077,21 @@ int plan_batch_passes(pac_plan_s* pl, long long copies, const long long* poff, c
   return PAC_SUCCESS;
 }
 int plan_bytes(pac_plan_s* pl) { return pl->main.bytes; }
+// the plan's waits report in *word (device memory of the caller's) from now on
+void plan_set_status_word(pac_plan_s* pl, int* word) { pl->status = word; }
+
+// Synchronise, read and clear a device status word.
+int check_status_word(int* status, const char* what, void* stream) {
+  int word = 0;
+  PAC_TRY(be_stream_sync(stream));
+  PAC_TRY(be_memcpy(&word, status, sizeof(int), CPY_D2H, stream));
+  PAC_TRY(be_stream_sync(stream));
+  if (word == PAC_SUCCESS) return PAC_SUCCESS;
+  PAC_TRY(be_memset(status, 0, sizeof(int), stream));
+  PAC_TRY(be_stream_sync(stream));
+  return set_error(word, "a bounded device wait of %s gave up (status %d); the output of the "
+                         "call it belongs to is incomplete", what, word);
+}
 // the factor lengths and stage radices of the plan (the autotuner skips a
 // knob set whose schedule it has already timed)
 std::string plan_signature(pac_plan_s* pl) {
@@ -1125,8 +1141,10 @@ static int build_schedule_in_arena(Schedule& s, int logn, int batch, Arena& ar, 
 
 int conv_in_scratch(void* scratch, size_t scratch_bytes, int logn, int batch, const double* x_re,
                     const double* x_im, const double* h_re, const double* h_im, double* y_re,
-                    double* y_im, void* stream) {
+                    double* y_im, int* status, long long wait_limit, void* stream) {
   pac_plan_s pl;
+  pl.status = status;
+  pl.wait_limit = wait_limit;
   pl.rank = 1;
   pl.dims[0] = 1 << logn;
   pl.logs[0] = logn;
@@ -1148,6 +1166,12 @@ int conv_in_scratch(void* scratch, size_t scratch_bytes, int logn, int batch, co
   return st;
 }
 
+}  // namespace pac
+
+namespace pac {
+// pac_noalloc.cu (the host replay: pac_emu.cpp): the status word of the
+// no-allocation entry point on the current device
+int noalloc_status_word(int** word);
 }  // namespace pac
 
 // ---------------------------------------------------------------------------
@@ -1512,15 +1536,14 @@ PAC_API int pac_plan_set_wait_limit(pac_plan_t plan, long long cycles) {
 
 PAC_API int pac_plan_check_status(pac_plan_t plan, pac_stream_t stream) {
   if (!plan) return set_error(PAC_ERROR_INVALID_VALUE, "pac_plan_check_status: NULL plan");
-  int word = 0;
-  PAC_TRY(be_stream_sync(stream));
-  PAC_TRY(be_memcpy(&word, plan->status, sizeof(int), CPY_D2H, stream));
-  PAC_TRY(be_stream_sync(stream));
-  if (word == PAC_SUCCESS) return PAC_SUCCESS;
-  PAC_TRY(be_memset(plan->status, 0, sizeof(int), stream));
-  PAC_TRY(be_stream_sync(stream));
-  return set_error(word, "a bounded device wait of this plan gave up (status %d); the output "
-                         "of the call it belongs to is incomplete", word);
+  return check_status_word(plan->status, "this plan", stream);
+}
+
+PAC_API int pac_noalloc_check_status(pac_stream_t stream) {
+  PAC_TRY(be_init());
+  int* word = nullptr;
+  PAC_TRY(noalloc_status_word(&word));
+  return check_status_word(word, "a no-allocation convolution", stream);
 }
 
 PAC_API const char* pac_status_string(int status) {

@@ -199,16 +199,19 @@ PAC_API int pac_convolve(pac_plan_t plan, const void* x_re, const void* x_im,
                          const void* hhat_re, const void* hhat_im, int hhat_per_problem,
                          void* y_re, void* y_im, double scale, pac_stream_t stream);
 
-/* Bounded device waits.  Kernels that wait on an mbarrier for their tensor
- * copies (the tensor-copy column passes, the opt-in pipelined column kernel)
- * give up after a limit of SM clock cycles instead of spinning forever: a
+/* Bounded device waits.  Kernels that wait on an mbarrier for their copies
+ * (the passes over rows of 32 to 8192 points, column passes of more than 256
+ * points and those of conj(A) on split axes, the tensor-copy and the opt-in
+ * pipelined column kernels) give up after a limit of SM clock cycles instead of spinning forever: a
  * CTA whose wait gives up writes PAC_ERROR_TIMEOUT into the plan's device
  * status word, issues nothing more, lets the copies it has in flight land
  * and leaves -- the output of that call is then incomplete, and the device
  * stays usable.  pac_plan_check_status synchronises `stream`, reads and
  * clears the status word and returns PAC_ERROR_TIMEOUT if a wait of any
  * call of this plan gave up since the last check (PAC_SUCCESS otherwise);
- * the fft.h functions check it after every call.  pac_plan_set_wait_limit
+ * the fft.h functions check it after every call.  A multi-plan has one word
+ * for all its shapes (pac_multi_check_status), pac_convolve_1d_noalloc one per
+ * device (pac_noalloc_check_status).  pac_plan_set_wait_limit
  * sets the limit, in SM cycles, for the plan's later calls (<= 0: the
  * default 2^31, about a second); a tiny limit makes the waits run out.
  * No counterpart in the reference (whose calls never wait on a device). */
@@ -238,6 +241,9 @@ PAC_API int pac_transform(pac_plan_t plan, int op, const void* in_re, const void
 PAC_API int pac_convolve_1d_noalloc(const double* x_re, const double* x_im, const double* h_re,
                                     const double* h_im, double* y_re, double* y_im, int n,
                                     int batch, pac_stream_t stream);
+/* As pac_plan_check_status, for the pac_convolve_1d_noalloc calls on the
+ * current device. */
+PAC_API int pac_noalloc_check_status(pac_stream_t stream);
 
 /* ---- Many convolutions of uneven shapes in one call ----------------------
  * No counterpart in the reference, which convolves one signal per call
@@ -307,6 +313,10 @@ PAC_API int pac_multi_create_tuned(pac_multi_t* multi, int nprob, const int* ran
 PAC_API int pac_multi_autotune(int nprob, const int* ranks, const int* dims, int digit_base,
                                int form, pac_stream_t stream, const char* cache_path,
                                pac_tune_result_t* result);
+/* As pac_plan_set_wait_limit and pac_plan_check_status, for the calls of a
+ * multi-plan (spectra and convolutions of every shape). */
+PAC_API int pac_multi_set_wait_limit(pac_multi_t multi, long long cycles);
+PAC_API int pac_multi_check_status(pac_multi_t multi, pac_stream_t stream);
 /* Level timing: while enabled, pac_multi_convolve issues the levels
  * directly (no graph), records a CUDA event around every level on the
  * caller's stream and waits for them (calls become synchronous);
