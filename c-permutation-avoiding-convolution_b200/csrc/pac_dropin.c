@@ -114,7 +114,9 @@ typedef struct {
 /*   entry, one copy in and one out per call;                               */
 /*   large entries: a pool of pinned slots, filled and emptied by a few      */
 /*   threads of the call.  One call at a time has the pool (others take the  */
-/*   driver's way); it exists while some large entry does.                  */
+/*   driver's way); it exists while some large entry does, so only entries   */
+/*   that hold a reference on it (pooled) may use it, and only for host      */
+/*   memory, which the threads read and write themselves.                    */
 /* ------------------------------------------------------------------------ */
 #define SMALL_BYTES (1 << 20)
 /* (1024 x 1024 calls: 4 threads of 1 MiB slots 2.8 ms, 8 of 512 KiB 3.3, 8 of
@@ -214,10 +216,13 @@ static void* copy_worker(void* arg) {
 
 /* both arrays of a pair between host and device (dev: re|im back to back),
  * in stream order; out: the host has them after finish() */
-static int copy_pair(double* dev, double* re, double* im, size_t nb, int in, pac_stream_t stream) {
+static int copy_pair(const entry_t* e, double* dev, double* re, double* im, size_t nb, int in,
+                     pac_stream_t stream) {
   int st;
-  const int direct = pac_host_kind(re) != 0 && pac_host_kind(im) != 0;
-  if (direct || !g_pool.pin || pthread_mutex_trylock(&g_pool.busy) != 0) {
+  const int kr = pac_host_kind(re), ki = pac_host_kind(im);
+  const int direct = kr != 0 && ki != 0;
+  if (direct || kr == 2 || ki == 2 || !e->pooled || !g_pool.pin ||
+      pthread_mutex_trylock(&g_pool.busy) != 0) {
     if (in) {
       st = pac_memcpy_h2d(dev, re, nb, stream);
       if (st == PAC_SUCCESS) st = pac_memcpy_h2d((char*)dev + nb, im, nb, stream);
@@ -398,8 +403,8 @@ static int arrays_in(entry_t* e, double* re, double* im, double* h_re, double* h
   const size_t nb = (size_t)e->N * sizeof(double);
   choose_staging(e, re, im, h_re, h_im);
   if (!e->staged) {
-    int st = copy_pair(e->x, re, im, nb, 1, e->s1);
-    if (st == PAC_SUCCESS && h_re) st = copy_pair(e->h, h_re, h_im, nb, 1, e->s1);
+    int st = copy_pair(e, e->x, re, im, nb, 1, e->s1);
+    if (st == PAC_SUCCESS && h_re) st = copy_pair(e, e->h, h_re, h_im, nb, 1, e->s1);
     return st;
   }
   memcpy(e->pin, re, nb);
@@ -413,7 +418,7 @@ static int arrays_in(entry_t* e, double* re, double* im, double* h_re, double* h
 /* a pair back: the first call for x, another for h */
 static int pair_out(entry_t* e, double* dev, double* re, double* im) {
   const size_t nb = (size_t)e->N * sizeof(double);
-  if (!e->staged) return copy_pair(dev, re, im, nb, 0, e->s1);
+  if (!e->staged) return copy_pair(e, dev, re, im, nb, 0, e->s1);
   return pac_memcpy_d2h(e->pin + (dev == e->x ? 0 : 2 * nb), dev, 2 * nb, e->s1);
 }
 /* waits; a device wait that gave up is reported; then a small entry's host
@@ -532,9 +537,9 @@ static void run_pac_conv(const char* fn, int rank, const int* dims, int r, doubl
     TRY(arrays_in(e, re, im, h_re, h_im));
     TRY(pac_transform(e->plan, PAC_OP_AT, hr, hi, hr, hi, e->s1));
   } else {
-    TRY(copy_pair(e->h, h_re, h_im, nb, 1, e->s1));
+    TRY(copy_pair(e, e->h, h_re, h_im, nb, 1, e->s1));
     TRY(pac_transform(e->plan, PAC_OP_AT, hr, hi, hr, hi, e->s1));
-    TRY(copy_pair(e->x, re, im, nb, 1, e->s2));
+    TRY(copy_pair(e, e->x, re, im, nb, 1, e->s2));
     TRY(pac_stream_wait_stream(e->s2, e->s1));
   }
   pac_stream_t s = e->staged ? e->s1 : e->s2;

@@ -16,6 +16,7 @@
 #include <atomic>
 #include <limits>
 #include <chrono>
+#include <mutex>
 #include <vector>
 
 #include "pac.h"
@@ -43,7 +44,25 @@ int be_free(void* p) {
 }
 int be_host_alloc(void** p, size_t bytes) { return be_malloc(p, bytes); }
 int be_host_free(void* p) { return be_free(p); }
-int be_host_kind(const void*) { return 0; }
+// Stand-ins for memory that the host does not own alone (pac_emu_device_array):
+// kind 2, reached by copies only; the host address itself holds other bytes
+struct DeviceArray {
+  char *lo, *hi, *shadow;
+};
+static std::mutex g_arrays_mu;
+static std::vector<DeviceArray> g_arrays;
+int be_host_kind(const void* p) {
+  std::lock_guard<std::mutex> g(g_arrays_mu);
+  for (const DeviceArray& a : g_arrays)
+    if ((const char*)p >= a.lo && (const char*)p < a.hi) return 2;
+  return 0;
+}
+static void* through_shadow(const void* p) {
+  std::lock_guard<std::mutex> g(g_arrays_mu);
+  for (const DeviceArray& a : g_arrays)
+    if ((const char*)p >= a.lo && (const char*)p < a.hi) return a.shadow + ((const char*)p - a.lo);
+  return const_cast<void*>(p);
+}
 int be_get_device() { return 0; }
 void be_set_device(int) {}
 int be_sync_event_create(void** ev) {
@@ -52,6 +71,8 @@ int be_sync_event_create(void** ev) {
 }
 int be_event_wait(void*) { return PAC_SUCCESS; }
 int be_memcpy(void* dst, const void* src, size_t bytes, int, void*) {
+  dst = through_shadow(dst);
+  src = through_shadow(src);
   if (bytes && dst != src) memmove(dst, src, bytes);
   return PAC_SUCCESS;
 }
@@ -785,6 +806,17 @@ int be_graph_destroy(void*) { return PAC_SUCCESS; }
 // read-only path since the library was loaded
 extern "C" PAC_API long long pac_emu_read_only_data_loads(void) {
   return pac::g_read_only_data.load();
+}
+
+// [host, host + bytes) stands for a device array whose bytes are at shadow
+// (shadow NULL: no longer)
+extern "C" PAC_API void pac_emu_device_array(void* host, size_t bytes, void* shadow) {
+  using namespace pac;
+  std::lock_guard<std::mutex> g(g_arrays_mu);
+  if (shadow) g_arrays.push_back({(char*)host, (char*)host + bytes, (char*)shadow});
+  else
+    for (size_t k = g_arrays.size(); k-- > 0;)
+      if (g_arrays[k].lo == (char*)host) g_arrays.erase(g_arrays.begin() + (long)k);
 }
 
 // read by the tests: dependent passes launched behind the filling of tables
