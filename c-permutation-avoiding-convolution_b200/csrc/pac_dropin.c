@@ -221,7 +221,9 @@ static int copy_pair(const entry_t* e, double* dev, double* re, double* im, size
   int st;
   const int kr = pac_host_kind(re), ki = pac_host_kind(im);
   const int direct = kr != 0 && ki != 0;
-  if (direct || kr == 2 || ki == 2 || !e->pooled || !g_pool.pin ||
+  /* (arrays that overlap are copied one after the other) */
+  const int apart = (char*)re + nb <= (char*)im || (char*)im + nb <= (char*)re;
+  if (direct || kr == 2 || ki == 2 || !apart || !e->pooled || !g_pool.pin ||
       pthread_mutex_trylock(&g_pool.busy) != 0) {
     if (in) {
       st = pac_memcpy_h2d(dev, re, nb, stream);
@@ -422,7 +424,8 @@ static int pair_out(entry_t* e, double* dev, double* re, double* im) {
   return pac_memcpy_d2h(e->pin + (dev == e->x ? 0 : 2 * nb), dev, 2 * nb, e->s1);
 }
 /* waits; a device wait that gave up is reported; then a small entry's host
- * arrays are written */
+ * arrays are written: the filter's first, as in a large call, so that an array
+ * that serves both ends as the signal's */
 static int finish(entry_t* e, double* re, double* im, double* h_re, double* h_im) {
   const size_t nb = (size_t)e->N * sizeof(double);
   int st = PAC_SUCCESS;
@@ -436,12 +439,12 @@ static int finish(entry_t* e, double* re, double* im, double* h_re, double* h_im
   if (e->plan) st = pac_host_fetch_status(e->plan, word, e->s1);
   if (st == PAC_SUCCESS) st = pac_stream_synchronize(e->s1);
   if (st != PAC_SUCCESS) return st;
-  memcpy(re, e->pin, nb);
-  memcpy(im, e->pin + nb, nb);
   if (h_re) {
     memcpy(h_re, e->pin + 2 * nb, nb);
     memcpy(h_im, e->pin + 3 * nb, nb);
   }
+  memcpy(re, e->pin, nb);
+  memcpy(im, e->pin + nb, nb);
   return *word == PAC_SUCCESS ? PAC_SUCCESS : pac_plan_check_status(e->plan, e->s1);
 }
 

@@ -1,7 +1,8 @@
 """Host arrays of the fft.h functions that are not plain memory of their own:
 a device or managed array beside ordinary ones (copied by the driver, never
 through the pinned slots that the copy threads read and write on the host), in
-small and large calls and while another shape holds the slots.
+small and large calls and while another shape holds the slots; arrays shared
+between the signal and the filter, whose last writer is the signal.
 
 On the host replay a "device" array is an address range whose bytes live
 elsewhere and that only copies reach; on the GPU it is managed memory."""
@@ -68,6 +69,23 @@ def check_mixed(L, shape, r, make):
                 assert np.abs(u.reshape(shape) - v).max() < 1e-9, (fn, which, k)
 
 
+def check_shared(L, shape, r):
+    """im and h_im are one array; then every array is the same one."""
+    g = rng(4)
+    for fn in ("permutation_avoiding_convolution", "fft_based_convolution"):
+        re, hr, zero = g.standard_normal(shape), g.standard_normal(shape), np.zeros(shape)
+        z = want(shape, r, [re, zero, hr, zero], fn)
+        im = zero.copy()
+        a, b = re.copy(), hr.copy()
+        call(L, fn, shape, r, [a, im, b, im])
+        for u, v in zip((a, im, b), (z[0], z[1], z[2])):
+            assert np.abs(u - v).max() < 1e-9, fn
+        z = want(shape, r, [re, re, re, re], fn)
+        a = re.copy()
+        call(L, fn, shape, r, [a] * 4)
+        assert np.abs(a - z[1]).max() < 1e-9, fn
+
+
 @pytest.mark.parametrize("shape,r", SHAPES)
 def test_mixed_replay(emu, shape, r):
     emu.pac_emu_device_array.argtypes = [C.c_void_p, C.c_size_t, C.c_void_p]
@@ -84,6 +102,11 @@ def test_mixed_replay(emu, shape, r):
     check_mixed(emu, shape, r, make)
 
 
+@pytest.mark.parametrize("shape,r", SHAPES)
+def test_shared_replay(emu, shape, r):
+    check_shared(emu, shape, r)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("shape,r", SHAPES)
 def test_mixed_gpu(lib, shape, r):
@@ -97,3 +120,9 @@ def test_mixed_gpu(lib, shape, r):
         return C.c_void_p(p), (lambda: view), (lambda: rt.cudaFree(p))
 
     check_mixed(lib, shape, r, make)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,r", SHAPES)
+def test_shared_gpu(lib, shape, r):
+    check_shared(lib, shape, r)
