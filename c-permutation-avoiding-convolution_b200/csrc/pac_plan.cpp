@@ -170,21 +170,27 @@ static bool builtin_split(const Schedule& s) {
          s.plane == 0 && getenv("PAC_MAX_FACTOR_LOG") == nullptr;
 }
 
-// the cheapest split of an axis of 2^lg, digit base 2^b2, into at most three
-// factors; rows: its last factor is the innermost of the plan.  Empty when
-// some factor would have no kernel (short axes, long axes of large bases).
-static std::vector<int> cheapest_split(int lg, int b2, bool rows, bool short_cols,
+// the cheapest split of an axis of 2^lg, digit base 2^b2, with 2^inner elements
+// of later axes between its neighbours, into at most three factors.  Empty when
+// some factor would have no kernel (short axes, long axes of large bases), and
+// when a column tile of the cheapest one would not fit its stride: beside an axis
+// of 2 or 4 points one pass over scalar elements is faster than more and
+// shorter factors that fit (1024 problems of 1024 x 2 FP32: 55 us against 88).
+static std::vector<int> cheapest_split(int lg, int b2, int inner, int bytes, bool short_cols,
                                        long long lines) {
   std::vector<int> best, cur;
   int best_cost = 1 << 30;
+  bool best_fits = false;
   VecGeo g;
-  auto cost = [&](int f, bool last) {
-    const bool row = rows && last;
+  // factor f at stride 2^logS
+  auto cost = [&](int f, int logS, bool last) {
+    const bool row = logS == 0;
     // one CTA takes 15 us for an 8192-point line: fewer lines than keep half
     // the SMs busy are faster in three passes of many tiles (one line 15 us
     // against 9.5)
     if (row && f == 13 && lines < 64) return 0;
-    if (f > 13 || (short_cols && !row && f > 8) || !vec_geometry(b2, row ? MODE_CONV : MODE_DIF, -1, f, row ? 0 : 1, &g)) return 0;
+    if (f > 13 || (short_cols && !row && f > 8)) return 0;
+    if (!vec_geometry(b2, row ? MODE_CONV : MODE_DIF, -1, f, row ? 0 : 1, &g)) return 0;
     return row ? kCostRow[f] : 2 * (last ? kCostCol[f] : kCostTw4[f]);
   };
   for (int n = 1; n <= 3; ++n)
@@ -198,17 +204,22 @@ static std::vector<int> cheapest_split(int lg, int b2, bool rows, bool short_col
         cur.clear();
         for (int f : {a, b, c})
           if (f > 0) cur.push_back(f);
-        int total = 0;
+        int total = 0, logS = inner + lg;
+        bool fits = true;
         for (size_t i = 0; i < cur.size() && total >= 0; ++i) {
-          const int v = cost(cur[i], i + 1 == cur.size());
+          logS -= cur[i];
+          const int v = cost(cur[i], logS, i + 1 == cur.size());
           total = v > 0 ? total + v : -1;
+          fits = fits && (logS == 0 || g.logW + (bytes == 8 ? 0 : 1) <= logS);
         }
         if (total > 0 && total < best_cost) {
           best_cost = total;
           best = cur;
+          best_fits = fits;
         }
         if (n < 2) break;
       }
+  if (!best_fits) best.clear();
   return best;
 }
 
@@ -217,9 +228,11 @@ static std::vector<int> cheapest_split(int lg, int b2, bool rows, bool short_col
 static int split_axes(Schedule& s, int rank, const int* logs, const int* b2s, int bytes,
                       long long batch, const Schedule* like = nullptr) {
   s.bytes = bytes;
-  // lines of the last axis (pairs of them in FP32)
+  // lines of the innermost axis (pairs of them in FP32)
   long long lines = batch;
-  for (int a = 0; a + 1 < rank; ++a) lines <<= logs[a];
+  int innermost = rank - 1;  // the last axis of more than one point
+  while (innermost > 0 && logs[innermost] == 0) --innermost;
+  for (int a = 0; a < innermost; ++a) lines <<= logs[a];
   lines = bytes == 8 ? lines : (lines + 1) / 2;
   s.b2 = b2s[rank - 1];
   if (like) s.vax = like->vax;
@@ -228,7 +241,9 @@ static int split_axes(Schedule& s, int rank, const int* logs, const int* b2s, in
     if (lg == 0) continue;
     const int b2 = b2s[a];
     if (builtin_split(s)) {
-      const std::vector<int> f = cheapest_split(lg, b2, a == rank - 1, s.short_cols, lines);
+      int inner = 0;
+      for (int i = a + 1; i < rank; ++i) inner += logs[i];
+      const std::vector<int> f = cheapest_split(lg, b2, inner, bytes, s.short_cols, lines);
       for (size_t i = 0; i < f.size(); ++i)
         s.vax.push_back({f[i], a, i == 0, i + 1 == f.size(), b2});
       if (!f.empty()) continue;
