@@ -771,6 +771,15 @@ static int run_transform(pac_plan_s* pl, const Schedule& s, int op, long long ba
   const long long N = pl->N;
   const int m = (int)s.vax.size();
   const long long total = batch * N;
+  // A x = swap(conj(A) swap(x)), swap exchanging real and imaginary parts: A
+  // takes the inverse kernels with the arrays exchanged (kernels over 8-byte
+  // elements; on the scalar ones of its own it took 62 us on 32 x 2^17 FP32
+  // where conj(A) takes 28, and was slower than with their longer factors)
+  if (op == PAC_OP_A || op == PAC_OP_UFFT) {
+    std::swap(in_re, in_im);
+    std::swap(out_re, out_im);
+    op = PAC_OP_CONJ_A;
+  }
   if (m == 0) {
     double sc = use_scale ? scale : 1.0;
     return be_scale_copy(total, s.bytes, in_re, in_im, out_re, out_im, sc, stream);
@@ -799,11 +808,10 @@ static int run_transform(pac_plan_s* pl, const Schedule& s, int op, long long ba
       passes.push_back(p);
     }
   } else {
-    int sign = (op == PAC_OP_A || op == PAC_OP_UFFT) ? -1 : +1;
     for (int vi = m - 1; vi >= 0; --vi) {
       PassSpec p = make_pass(s, vi, batch, N);
       p.d.mode = MODE_DIT;
-      p.d.sign = sign;
+      p.d.sign = +1;
       p.d.tw4 = s.vax[vi].last ? 0 : 2;
       passes.push_back(p);
     }

@@ -61,8 +61,8 @@ namespace pac {
 #define PAC_VEC_SMALL(X) X(1, 1) X(1, 2) X(1, 3) X(1, 4) X(2, 2) X(2, 4) X(3, 3)
 
 // The modes and signs that a pass of a factor can have: forward (A^T, FFT),
-// the inverse FFT's DIF, conj(A), and the fused convolution (rows).  (A,
-// a DIT of sign -1, stays on the generic kernel.)
+// the inverse FFT's DIF, conj(A), and the fused convolution (rows).  (A is
+// conj(A) with real and imaginary parts exchanged.)
 inline bool vec_mode(int mode, int sign, int cols) {
   if (mode == MODE_CONV) return !cols;
   return mode == MODE_DIF || (mode == MODE_DIT && sign > 0);
