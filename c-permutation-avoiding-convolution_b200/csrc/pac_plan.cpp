@@ -165,9 +165,39 @@ static const int kCostRow[14] = {0, 0, 0, 0, 0, 100, 96, 98, 98, 123, 130, 144, 
 static const int kCostCol[14] = {0, 84, 84, 84, 85, 87, 88, 90, 92, 101, 124, 140, 0, 0};
 static const int kCostTw4[14] = {0, 90, 90, 90, 112, 92, 93, 97, 102, 108, 137, 165, 0, 0};
 
+// The environment's kernel choices, looked up once per call (one getenv per
+// choice and pass took 1 us of a call's 5).  PAC_PIPE=0 and
+// PAC_SPECIAL_VARIANT=0 are the built-in choices, as if unset (PAC_COLTMA=0, no
+// tensor copies, and PAC_CLUSTER_VARIANT=0, its first candidate, are not).
+struct EnvChoice {
+  const char *coltma = nullptr, *pipe = nullptr, *cluster = nullptr, *special = nullptr;
+  // the passes run on the kernels over scalar elements
+  bool scalar() const { return coltma || pipe || cluster || special; }
+};
+static EnvChoice env_choice() {
+  EnvChoice c;
+  for (char** e = environ; e && *e; ++e) {
+    const char* v = *e;
+    if (v[0] != 'P' || v[1] != 'A' || v[2] != 'C' || v[3] != '_') continue;
+    auto is = [&](const char* name, const char** to) {
+      const size_t n = strlen(name);
+      if (strncmp(v + 4, name, n) == 0 && v[4 + n] == '=') *to = v + 5 + n;
+    };
+    is("COLTMA", &c.coltma);
+    is("PIPE", &c.pipe);
+    is("CLUSTER_VARIANT", &c.cluster);
+    is("SPECIAL_VARIANT", &c.special);
+  }
+  if (c.pipe && atoi(c.pipe) == 0) c.pipe = nullptr;
+  if (c.special && atoi(c.special) == 0) c.special = nullptr;
+  return c;
+}
+
+// (under a kernel choice of the environment too the factors are those that the
+// scalar kernels want: 64 FP64 lines of 2^16 points 96 us, 141 with these)
 static bool builtin_split(const Schedule& s) {
   return !s.tc && s.flog_cap == 0 && s.rlog_cap >= 4 && s.special == 0 && s.w_shift == 0 &&
-         s.plane == 0 && getenv("PAC_MAX_FACTOR_LOG") == nullptr;
+         s.plane == 0 && getenv("PAC_MAX_FACTOR_LOG") == nullptr && !env_choice().scalar();
 }
 
 // the cheapest split of an axis of 2^lg, digit base 2^b2, with 2^inner elements
@@ -497,28 +527,6 @@ static PassSpec make_pass(const Schedule& s, int vi, long long batch, long long 
   return p;
 }
 
-// The environment's kernel choices, looked up once per call (one getenv per
-// choice and pass took 1 us of a call's 5)
-struct EnvChoice {
-  const char *coltma = nullptr, *pipe = nullptr, *cluster = nullptr, *special = nullptr;
-};
-static EnvChoice env_choice() {
-  EnvChoice c;
-  for (char** e = environ; e && *e; ++e) {
-    const char* v = *e;
-    if (v[0] != 'P' || v[1] != 'A' || v[2] != 'C' || v[3] != '_') continue;
-    auto is = [&](const char* name, const char** to) {
-      const size_t n = strlen(name);
-      if (strncmp(v + 4, name, n) == 0 && v[4 + n] == '=') *to = v + 5 + n;
-    };
-    is("COLTMA", &c.coltma);
-    is("PIPE", &c.pipe);
-    is("CLUSTER_VARIANT", &c.cluster);
-    is("SPECIAL_VARIANT", &c.special);
-  }
-  return c;
-}
-
 // Switch a pass to the kernel over 8-byte elements (pac_vec.cuh) of its
 // geometry.  Plans with knobs and the environment's kernel choices keep the
 // kernels those select; a column tile has to
@@ -531,7 +539,7 @@ static bool apply_vec(const Schedule& s, PassSpec& p, const EnvChoice& env) {
   if (d.tc)
     for (int i = 0; i < d.nst; ++i)
       if (d.rlog[i] == 4) return false;
-  if (env.coltma || env.pipe || env.cluster || env.special) return false;
+  if (env.scalar()) return false;
   const int cols = d.logS > 0 ? 1 : 0;
   VecGeo g;
   if (!vec_geometry(p.b2, d.mode, d.sign, d.logL, cols, &g)) return false;
@@ -592,7 +600,7 @@ static void apply_special(const Schedule& s, PassSpec& p, const EnvChoice& env) 
   // SM, tensor-copy prefetch of the next tile (16-byte aligned input arrays
   // for the tensor maps)
   const char* pipe = d.tc || s.rlog_cap < 4 ? nullptr : env.pipe;
-  if (d.logS > 0 && cvar == nullptr && pipe != nullptr && atoi(pipe) != 0 &&
+  if (d.logS > 0 && cvar == nullptr && pipe != nullptr &&
       pipe_geometry(s.bytes, p.b2, d.mode, d.sign, d.logL, &logW, &nt) && logW <= d.logS &&
       (d.nlines & ((1LL << logW) - 1)) == 0 && (d.nlines >> d.logS) < (1LL << 31) &&
       ((uintptr_t)d.in_re | (uintptr_t)d.in_im) % 16 == 0) {
