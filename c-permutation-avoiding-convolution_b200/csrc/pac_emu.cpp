@@ -819,6 +819,12 @@ extern "C" PAC_API void pac_emu_device_array(void* host, size_t bytes, void* sha
       if (g_arrays[k].lo == (char*)host) g_arrays.erase(g_arrays.begin() + (long)k);
 }
 
+// the shared memory that a launch over 8-byte elements asks for
+extern "C" PAC_API size_t pac_emu_vec_smem(size_t smem, long long tiles, long long fit, int sms,
+                                           int legacy_stream) {
+  return pac::vec_smem(smem, tiles, fit, sms, legacy_stream != 0);
+}
+
 // read by the tests: dependent passes launched behind the filling of tables
 // that nothing had waited for
 extern "C" PAC_API long long pac_emu_early_tables(void) { return pac::g_early_tables.load(); }

@@ -33,9 +33,6 @@ constexpr int kBytes = 4;
 #define PAC_VEC_MINB(M8, M4) M4
 #endif
 
-// shared memory of an SM, and the most that a CTA may ask for (static kept)
-constexpr size_t kSmemSM = 228 * 1024, kSmemCTA = 226 * 1024;
-
 // CTAs that fit the device with this kernel, its shared-memory limit raised
 // (once per kernel and device)
 struct Resident {
@@ -52,7 +49,7 @@ int resident(Resident& r, K kern, int nt, size_t smem, long long* out) {
     *out = r.ctas[dev];
     return PAC_SUCCESS;
   }
-  PAC_CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCTA),
+  PAC_CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVecSmemCTA),
          "cudaFuncSetAttribute");
   int nb = 0, sms = 0;
   PAC_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, nt, smem),
@@ -68,10 +65,8 @@ int resident(Resident& r, K kern, int nt, size_t smem, long long* out) {
 // A launch that may overlap the end of the work before it in the stream: the
 // kernels set up (barriers, twiddles in shared memory) and then wait for that
 // work (pdl_wait).  slots: CTAs that fit the device (negative: a CTA a tile,
-// else persistent CTAs; 0 unknown).  Fewer tiles than that have to be spread
-// over the SMs: CTAs that arrive while the kernel before still runs would
-// otherwise pile up on the SMs that it leaves first, so each reserves its
-// share of an SM's shared memory.
+// else persistent CTAs; 0 unknown); fewer tiles than that may reserve shared
+// memory (vec_smem).
 // (A pass that may not start early, PassDesc.dependent, is launched plainly.)
 template <class K, class... A>
 int pdl_launch(K kern, long long tiles, long long slots, int nt, size_t smem, cudaStream_t st,
@@ -79,12 +74,7 @@ int pdl_launch(K kern, long long tiles, long long slots, int nt, size_t smem, cu
   const long long fit = slots < 0 ? -slots : slots;
   long long grid = tiles;
   if (slots > 0 && tiles > slots) grid = slots;
-  if (fit > 0 && tiles < fit) {
-    const int sms = be_num_sms();
-    const long long per_sm = (tiles + sms - 1) / sms;
-    const size_t share = (size_t)(kSmemSM / per_sm) / 1024 * 1024 - 2048;
-    if (share > smem) smem = share < kSmemCTA ? share : kSmemCTA;
-  }
+  smem = vec_smem(smem, tiles, fit, be_num_sms(), st == nullptr || st == cudaStreamLegacy);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)nt);

@@ -80,6 +80,26 @@ PAC_HDC bool vec_direct(int mode, int logL, int tw4) {
   return logL <= 8 && !(mode == MODE_DIT && tw4);
 }
 
+// Dynamic shared memory of a launch of `tiles` CTAs of which `fit` fit the
+// device.  On one stream fewer tiles than that are better spread over the SMs:
+// CTAs that arrive while the kernel before still runs would otherwise pile up on
+// the SMs that it leaves first, so each reserves its share of an SM's shared
+// memory (1024 x 1024 FP32 21.6 us against 24.0, 64^3 FP64 14.2 against 17.0).
+// But a reserved SM takes no CTA of another stream's either: eight plans on
+// eight streams took 30.0 us a call with it against 18.6 (256 x 256 FP64), 122
+// against 76 (8 x 2^16), more than the scalar kernels (20.6, 83).  So only
+// launches on the legacy default stream, which other streams do not run beside
+// unless they were made not to wait for it, reserve.
+constexpr size_t kVecSmemSM = 228 * 1024;   // of an SM
+constexpr size_t kVecSmemCTA = 226 * 1024;  // the most that a CTA may ask for (static kept)
+inline size_t vec_smem(size_t smem, long long tiles, long long fit, int sms, bool legacy_stream) {
+  if (!legacy_stream || fit <= 0 || tiles >= fit) return smem;
+  const long long per_sm = (tiles + sms - 1) / sms;
+  const size_t share = kVecSmemSM / (size_t)per_sm / 1024 * 1024 - 2048;
+  if (share <= smem) return smem;
+  return share < kVecSmemCTA ? share : kVecSmemCTA;
+}
+
 struct VecGeo {
   int logW = 0, nt = 0;
   size_t smem = 0;
