@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(NT, MINB) pac_vec_direct_kernel(const __grid_c
 
 template <class V, int B2, int MODE, int SIGN, int LOGL, int TW4, int OFFS>
 __global__ void __launch_bounds__(256) pac_vec_small_kernel(const __grid_constant__ PassDesc d) {
-  const long long u = (long long)blockIdx.x * 256 + threadIdx.x;
+  const long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   pdl_wait();
   if (u < d.nlines / VT<V>::LPU)
     VecSmall<V, B2, MODE, SIGN, LOGL, OFFS>::template run<TW4>(d, u, [] { pdl_trigger(); });
