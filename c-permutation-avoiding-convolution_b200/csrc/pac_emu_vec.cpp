@@ -67,7 +67,8 @@ int rows_as(const PassDesc& d) {
   for (long long tile = 0; tile < tiles; ++tile) {
     nan_fill<VP>(buf);
     const long long g0 = tile * wl, n = std::min(wl, d.nlines - g0) << LOGL;
-    for (long long l = 0; l < n >> LOGL; ++l) {
+    for (int t = 0; t < NT && d.unaligned; ++t) VP::copy_in(d, tile, t, buf.data());
+    for (long long l = 0; l < n >> LOGL && !d.unaligned; ++l) {
       const long long o = VP::line_off(d, g0 + l);
       std::copy_n((const Real*)d.in_re + o, VP::L, (Real*)D + (l << LOGL));
       std::copy_n((const Real*)d.in_im + o, VP::L, (Real*)(D + VP::DIM) + (l << LOGL));
@@ -105,7 +106,8 @@ int cols_as(const PassDesc& d) {
     nan_fill<VP>(buf);
     int i0 = 0, o = 0;
     if (!VP::DIRECT) VP::tile_coords(d, tile, i0, o);
-    for (int e = 0; e < VP::L && !VP::DIRECT; ++e)
+    for (int t = 0; t < T && d.unaligned && !VP::DIRECT; ++t) VP::copy_in(d, tile, t, buf.data());
+    for (int e = 0; e < VP::L && !VP::DIRECT && !d.unaligned; ++e)
       for (int w = 0; w < VP::W; ++w) {
         const long long gi = ((long long)o << (LOGL + su)) + ((long long)e << su) + i0 + w;
         D[(e << LOGW) + w] = ire[gi];

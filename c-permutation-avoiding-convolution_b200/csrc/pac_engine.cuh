@@ -117,6 +117,9 @@ struct PassDesc {
   // 2^porder_logR positions transposed) in elements of porder bytes; 0: no
   int porder;
   int porder_logR;
+  // vec passes: 1: an array does not start at a multiple of 16 bytes, so the
+  // threads of a CTA copy its tiles in
+  int unaligned;
   // vec passes: the launch may start while the work queued ahead of it still
   // runs, and then reads its twiddle tables at once.  Only where those were
   // complete before that work began: the tables of a plan that was handed out,

@@ -143,9 +143,11 @@ int cols_copied(const PassDesc& d, cudaStream_t st) {
   long long slots = 0;
   int s = resident(res, kern, T, VP::SMEM + 128, &slots);
   if (s != PAC_SUCCESS || d.vec == VEC_PREPARE) return s;
-  CUtensorMap m[2];
-  if ((s = col_map<VP>(&m[0], d.in_re, d)) != PAC_SUCCESS) return s;
-  if ((s = col_map<VP>(&m[1], d.in_im, d)) != PAC_SUCCESS) return s;
+  CUtensorMap m[2] = {};
+  if (!d.unaligned) {
+    if ((s = col_map<VP>(&m[0], d.in_re, d)) != PAC_SUCCESS) return s;
+    if ((s = col_map<VP>(&m[1], d.in_im, d)) != PAC_SUCCESS) return s;
+  }
   const long long tiles = (d.nlines / VP::LPU) >> LOGW;
   if (tiles > 4 * slots) {
     // rounds enough to hide a launch; as a dependent launch these wide CTAs

@@ -832,6 +832,36 @@ struct VecPass {
     return d.poff[l >> d.logLP] + ((l & ((1LL << d.logLP) - 1)) << LOGL);
   }
 
+  // ---- the dense tile of a pass whose arrays the copies cannot take ------------
+  static PAC_HD void copy_in(const PassDesc& d, long long tile, int t, CV<V>* B) {
+    if constexpr (COLS) {
+      const long long base = tile_base(d, tile);
+      const int rowsh = d.logS - ilog2(LPU);
+      V* D = reinterpret_cast<V*>(B);
+#if defined(__CUDACC__)
+#pragma unroll 4
+#endif
+      for (int q = t; q < DIM; q += NT) {
+        const long long gi = base + ((long long)(q >> LOGW) << rowsh) + (q & (W - 1));
+        D[q] = ld_data((const V*)d.in_re + gi);
+        D[DIM + q] = ld_data((const V*)d.in_im + gi);
+      }
+    } else {
+      constexpr long long WL = W * LPU;
+      const long long g0 = tile * WL, left = d.nlines - g0;
+      const int n = (int)(left < WL ? left : WL) << LOGL;
+      Real* D = reinterpret_cast<Real*>(B);
+#if defined(__CUDACC__)
+#pragma unroll 4
+#endif
+      for (int q = t; q < n; q += NT) {
+        const long long gi = line_off(d, g0 + (q >> LOGL)) + (q & (L - 1));
+        D[q] = ld_data((const Real*)d.in_re + gi);
+        D[LPU * DIM + q] = ld_data((const Real*)d.in_im + gi);
+      }
+    }
+  }
+
   // ---- DIT rows: the dense tile through registers into the padded layout --
   static PAC_HD void relay_read(int t, const CV<V>* B, CV<V> (&x)[TPT]) {
     const V* D = reinterpret_cast<const V*>(B);

@@ -36,6 +36,7 @@ struct VecExec {
   CV<V> x[VP::TPT];
   typename VP::Mid m;
   long long next, ntiles;
+  bool copies;
   Issue& issue;
   template <class F>
   __device__ __forceinline__ void each(F&& f) {
@@ -52,7 +53,7 @@ struct VecExec {
     fence_proxy_async();
     sync();
     if (next >= ntiles) pdl_trigger();
-    else if (threadIdx.x == 0) issue(next);
+    else if (threadIdx.x == 0 && copies) issue(next);
   }
 };
 
@@ -71,12 +72,18 @@ __device__ __forceinline__ void vec_tiles(const PassDesc& d, CV<V>* B, uint64_t*
   pdl_wait();
   __syncthreads();
   long long tile = blockIdx.x;
-  if (threadIdx.x == 0 && tile < ntiles) issue(tile);
+  if (threadIdx.x == 0 && tile < ntiles && !d.unaligned) issue(tile);
   uint32_t phase = 0;
-  VecExec<VP, V, Issue> ex{{}, {}, tile, ntiles, issue};
+  VecExec<VP, V, Issue> ex{{}, {}, tile, ntiles, !d.unaligned, issue};
   for (; tile < ntiles; tile += gridDim.x) {
     ex.next = tile + gridDim.x;
-    const bool ok = mbar_wait_bounded(bar, phase, wait_limit_of(d));
+    bool ok = true;
+    if (d.unaligned) {
+      VP::copy_in(d, tile, threadIdx.x, B);
+      vec_sync<VP::kThreads>();  // (a vote alone orders no memory accesses)
+    } else {
+      ok = mbar_wait_bounded(bar, phase, wait_limit_of(d));
+    }
     if (!vec_all<VP::kThreads>(ok)) {
       // a wait gave up: report it, issue nothing more, keep the CTA (its
       // shared memory) alive until the copy in flight has landed
