@@ -488,6 +488,7 @@ int be_malloc(void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
   if (e != cudaSuccess) {
     *p = nullptr;
+    cudaGetLastError();  // (told here; not by the next launch's check)
     return set_error(PAC_ERROR_ALLOC, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
   }
   return PAC_SUCCESS;
@@ -502,6 +503,7 @@ int be_host_alloc(void** p, size_t bytes) {
   cudaError_t e = cudaHostAlloc(p, bytes ? bytes : 16, cudaHostAllocPortable);
   if (e != cudaSuccess) {
     *p = nullptr;
+    cudaGetLastError();
     return set_error(PAC_ERROR_ALLOC, "cudaHostAlloc(%zu): %s", bytes, cudaGetErrorString(e));
   }
   return PAC_SUCCESS;

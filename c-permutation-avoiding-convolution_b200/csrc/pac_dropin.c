@@ -94,9 +94,11 @@ typedef struct {
   long long N;
   pac_plan_t plan; /* NULL for shapes the butterflies do not run on */
   double *x, *h;   /* device: x re|im, h re|im, each 2N doubles, back to back */
-  double* hhat;    /* device: 2N doubles, the plan-order spectrum */
+  double* hhat;    /* device: 2N doubles, the plan-order spectrum; NULL where
+                      memory is short: h is reordered in place */
   int* rho;        /* device: N ints (permutation-only paths) */
-  char* pin;       /* pinned: staging of a small entry's arrays, status word */
+  char* pin;       /* pinned: staging of a small entry's arrays, status word;
+                      NULL: its arrays go the driver's way */
   int pooled;      /* a large entry: holds a reference on the staging pool */
   int staged;      /* this call goes through pin */
   pac_stream_t s1, s2;
@@ -296,12 +298,19 @@ static int entry_fill(entry_t* e, int rank, const int* dims, int r, int want_pla
   for (int a = 0; a < rank; ++a) e->N *= dims[a];
   int st = PAC_SUCCESS;
   if (want_plan) st = pac_plan_create(&e->plan, rank, dims, 1, r, PAC_FORM_F64);
-  if (st == PAC_SUCCESS) st = pac_malloc((void**)&e->x, (size_t)e->N * 48);
+  int third = 1;
+  if (st == PAC_SUCCESS) {
+    st = pac_malloc((void**)&e->x, (size_t)e->N * 48);
+    if (st == PAC_ERROR_ALLOC) {
+      third = 0;
+      st = pac_malloc((void**)&e->x, (size_t)e->N * 32);
+    }
+  }
   if (st == PAC_SUCCESS) {
     e->h = e->x + 2 * e->N;
-    e->hhat = e->h + 2 * e->N;
+    e->hhat = third ? e->h + 2 * e->N : NULL;
     if ((size_t)e->N * 32 <= SMALL_BYTES) {
-      st = pac_host_alloc((void**)&e->pin, (size_t)e->N * 32 + 64);
+      if (pac_host_alloc((void**)&e->pin, (size_t)e->N * 32 + 64) != PAC_SUCCESS) e->pin = NULL;
     } else {
       pool_hold();
       e->pooled = 1;
@@ -543,12 +552,15 @@ static void run_pac_conv(const char* fn, int rank, const int* dims, int r, doubl
     TRY(copy_pair(e, e->h, h_re, h_im, nb, 1, e->s1));
     TRY(pac_transform(e->plan, PAC_OP_AT, hr, hi, hr, hi, e->s1));
     TRY(copy_pair(e, e->x, re, im, nb, 1, e->s2));
-    TRY(pac_stream_wait_stream(e->s2, e->s1));
   }
+  /* (in place: A^T h leaves first) */
+  double* H = e->hhat ? e->hhat : e->h;
+  if (!e->hhat) TRY(pair_out(e, e->h, h_re, h_im));
+  if (!e->staged) TRY(pac_stream_wait_stream(e->s2, e->s1));
   pac_stream_t s = e->staged ? e->s1 : e->s2;
-  TRY(pac_spectrum_to_plan_order(e->plan, hr, hi, 1, e->hhat, e->hhat + N, 1.0, s));
-  TRY(pac_convolve(e->plan, xr, xi, e->hhat, e->hhat + N, 0, xr, xi, 1.0 / (double)N, s));
-  TRY(pair_out(e, e->h, h_re, h_im));
+  TRY(pac_spectrum_to_plan_order(e->plan, hr, hi, 1, H, H + N, 1.0, s));
+  TRY(pac_convolve(e->plan, xr, xi, H, H + N, 0, xr, xi, 1.0 / (double)N, s));
+  if (e->hhat) TRY(pair_out(e, e->h, h_re, h_im));
   if (!e->staged) TRY(pac_stream_wait_stream(e->s1, e->s2));
   TRY(pair_out(e, e->x, re, im));
   TRY(finish(e, re, im, h_re, h_im));

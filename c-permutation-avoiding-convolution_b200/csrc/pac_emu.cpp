@@ -33,7 +33,12 @@ int be_init() { return PAC_SUCCESS; }
 // a few "SMs", so that persistent kernels replay CTAs that walk several tiles
 int be_num_sms() { return 3; }
 
+// allocations larger than these fail (pac_emu_alloc_limits; 0: none does)
+static std::atomic<size_t> g_most_device{0}, g_most_pinned{0};
 int be_malloc(void** p, size_t bytes) {
+  *p = nullptr;
+  if (g_most_device && bytes > g_most_device)
+    return set_error(PAC_ERROR_ALLOC, "the replay's device memory is limited");
   *p = aligned_alloc(256, ((bytes ? bytes : 16) + 255) / 256 * 256);
   if (!*p) return set_error(PAC_ERROR_ALLOC, "host allocation failed");
   return PAC_SUCCESS;
@@ -42,7 +47,12 @@ int be_free(void* p) {
   free(p);
   return PAC_SUCCESS;
 }
-int be_host_alloc(void** p, size_t bytes) { return be_malloc(p, bytes); }
+int be_host_alloc(void** p, size_t bytes) {
+  *p = nullptr;
+  if (g_most_pinned && bytes > g_most_pinned)
+    return set_error(PAC_ERROR_ALLOC, "the replay's pinned memory is limited");
+  return be_malloc(p, bytes);
+}
 int be_host_free(void* p) { return be_free(p); }
 // Stand-ins for memory that the host does not own alone (pac_emu_device_array):
 // kind 2, reached by copies only; the host address itself holds other bytes
@@ -817,6 +827,12 @@ extern "C" PAC_API void pac_emu_device_array(void* host, size_t bytes, void* sha
   else
     for (size_t k = g_arrays.size(); k-- > 0;)
       if (g_arrays[k].lo == (char*)host) g_arrays.erase(g_arrays.begin() + (long)k);
+}
+
+// the largest device and pinned allocation that succeeds (0: any)
+extern "C" PAC_API void pac_emu_alloc_limits(size_t device, size_t pinned) {
+  pac::g_most_device = device;
+  pac::g_most_pinned = pinned;
 }
 
 // the shared memory that a launch over 8-byte elements asks for

@@ -355,7 +355,27 @@ static int build_tables(Schedule& s, Arena* ar, void* stream, size_t extra = 0) 
     size_t need = extra;
     for (const Piece& p : pieces) need += (p.bytes + 255) & ~(size_t)255;
     if (need == 0) return PAC_SUCCESS;
-    PAC_TRY(be_malloc(&s.block, need));
+    int st = be_malloc(&s.block, need);
+    if (st == PAC_ERROR_ALLOC) {
+      // without the whole 4-step tables, which only make passes faster
+      size_t less = extra;
+      std::vector<Piece> kept;
+      for (const Piece& p : pieces) {
+        bool whole = false;
+        for (auto& kv : s.tw4)
+          for (auto& f : kv.second.tab) whole = whole || p.to == &f.second;
+        if (whole) continue;
+        kept.push_back(p);
+        less += (p.bytes + 255) & ~(size_t)255;
+      }
+      if (less < need) {
+        pieces = kept;
+        need = less;
+        for (auto& kv : s.tw4) kv.second.tab.clear();
+        st = be_malloc(&s.block, need);
+      }
+    }
+    PAC_TRY(st);
     if (extra) PAC_TRY(be_memset(s.block, 0, extra, stream));
     own = {(char*)s.block + extra, (char*)s.block + need};
     ar = &own;
