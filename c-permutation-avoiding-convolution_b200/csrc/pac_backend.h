@@ -24,7 +24,7 @@ int be_host_free(void* p);
 int be_host_kind(const void* p);  // 0 ordinary, 1 pinned, 2 device or managed
 int be_get_device();
 void be_set_device(int device);
-int be_sync_event_create(void** ev);  // no timing, its waiter sleeps
+int be_sync_event_create(void** ev);  // no timing (its waiter spins; a sleeping one was no faster)
 int be_event_wait(void* ev);
 int be_memcpy(void* dst, const void* src, size_t bytes, int kind, void* stream);
 int be_memset(void* dst, int value, size_t bytes, void* stream);

@@ -27,7 +27,7 @@
 //
 // The member functions are per-thread work between two CTA barriers; the
 // sm_100a kernel (pac_vec_kernel.cuh) puts __syncthreads() between them, the
-// host replay (pac_emu.cpp) runs each for every thread in turn.
+// host replay (pac_emu_vec.cpp) runs each for every thread in turn.
 #pragma once
 
 namespace pac {

@@ -210,10 +210,10 @@ PAC_API int pac_convolve(pac_plan_t plan, const void* x_re, const void* x_im,
 /* Bounded device waits.  Kernels that wait on an mbarrier for their copies
  * (the passes over rows of 32 to 8192 points, column passes of more than 256
  * points and those of conj(A) on split axes, the tensor-copy and the opt-in
- * pipelined column kernels) give up after a limit of SM clock cycles instead of spinning forever: a
- * CTA whose wait gives up writes PAC_ERROR_TIMEOUT into the plan's device
- * status word, issues nothing more, lets the copies it has in flight land
- * and leaves -- the output of that call is then incomplete, and the device
+ * pipelined column kernels) give up after a limit of SM clock cycles instead
+ * of spinning forever: a CTA whose wait gives up writes PAC_ERROR_TIMEOUT into
+ * the plan's device status word, issues nothing more, lets the copies it has in
+ * flight land and leaves -- the output of that call is then incomplete, and the device
  * stays usable.  pac_plan_check_status synchronises `stream`, reads and
  * clears the status word and returns PAC_ERROR_TIMEOUT if a wait of any
  * call of this plan gave up since the last check (PAC_SUCCESS otherwise);
