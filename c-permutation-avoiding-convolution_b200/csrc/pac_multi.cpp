@@ -49,7 +49,8 @@ int plan_batch_passes(pac_plan_s* pl, long long copies, const long long* poff, c
                       void* y_im, std::vector<PassDesc>& descs, std::vector<long long>& tiles);
 void plan_set_status_word(pac_plan_s* pl, int* word);
 int check_status_word(int* status, const char* what, void* stream);
-int plan_create_for_batch(pac_plan_t* plan, int rank, const int* dims, const int* bases, int form);
+int plan_create_for_batch(pac_plan_t* plan, int rank, const int* dims, const int* bases, int form,
+                          int cached);
 }  // namespace pac
 
 using namespace pac;
@@ -396,8 +397,12 @@ static int create_multi(pac_multi_t* multi, int nprob, const int* ranks, const i
     if (it == seen.end()) {
       pac_plan_t pl = nullptr;
       const int bases[3] = {digit_base, digit_base, digit_base};
-      int st = tune ? pac_plan_create_tuned(&pl, r, key.data(), bases, 1, form, tune)
-                    : plan_create_for_batch(&pl, r, key.data(), bases, form);
+      // (knobs of 0 are the built-in choices of a multi-plan: the tuner starts
+      // from them)
+      int st = tune && (tune->max_factor_log || tune->max_radix_log || tune->special ||
+                        tune->w_shift || tune->plane)
+                   ? pac_plan_create_tuned(&pl, r, key.data(), bases, 1, form, tune)
+                   : plan_create_for_batch(&pl, r, key.data(), bases, form, tune == nullptr);
       if (st != PAC_SUCCESS) return st;
       it = seen.emplace(key, (int)m->plans.size()).first;
       m->plans.push_back(pl);

@@ -1350,12 +1350,12 @@ PAC_API int pac_plan_create(pac_plan_t* plan, int rank, const int* dims, int bat
 
 }  // extern "C"
 namespace pac {
-// a multi-plan's plan of one shape: the built-in knobs (or the cached ones),
-// factors whose passes can serve problems at any offset
-int plan_create_for_batch(pac_plan_t* plan, int rank, const int* dims, const int* bases,
-                          int form) {
+// a multi-plan's plan of one shape: the built-in knobs (or, with `cached`, those
+// of the tuning cache), factors whose passes can serve problems at any offset
+int plan_create_for_batch(pac_plan_t* plan, int rank, const int* dims, const int* bases, int form,
+                          int cached) {
   pac_tune_t t;
-  if (tune_from_env_cache(rank, dims, bases, 1, form, &t))
+  if (cached && tune_from_env_cache(rank, dims, bases, 1, form, &t))
     return create_plan(plan, rank, dims, bases, 1, form, &t);
   return create_plan(plan, rank, dims, bases, 1, form, nullptr, 1);
 }
