@@ -17,6 +17,8 @@
 #include <limits>
 #include <chrono>
 #include <mutex>
+#include <set>
+#include <thread>
 #include <vector>
 
 #include "pac.h"
@@ -74,7 +76,13 @@ static void* through_shadow(const void* p) {
   return const_cast<void*>(p);
 }
 int be_get_device() { return 0; }
-void be_set_device(int) {}
+// the threads that copy host arrays (each sets its device)
+static std::mutex g_copiers_mu;
+static std::set<std::thread::id> g_copiers;
+void be_set_device(int) {
+  std::lock_guard<std::mutex> g(g_copiers_mu);
+  g_copiers.insert(std::this_thread::get_id());
+}
 int be_sync_event_create(void** ev) {
   *ev = new double(0.0);
   return PAC_SUCCESS;
@@ -833,6 +841,14 @@ extern "C" PAC_API void pac_emu_device_array(void* host, size_t bytes, void* sha
 extern "C" PAC_API void pac_emu_alloc_limits(size_t device, size_t pinned) {
   pac::g_most_device = device;
   pac::g_most_pinned = pinned;
+}
+
+// threads that have copied host arrays since the last call of this
+extern "C" PAC_API int pac_emu_copy_threads(void) {
+  std::lock_guard<std::mutex> g(pac::g_copiers_mu);
+  const int n = (int)pac::g_copiers.size();
+  pac::g_copiers.clear();
+  return n;
 }
 
 // the shared memory that a launch over 8-byte elements asks for
